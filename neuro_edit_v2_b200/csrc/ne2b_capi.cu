@@ -153,7 +153,7 @@ static ne2b_status create_from_list(ne2b::Engine &eng, const ne2b_net_desc *net,
     dc.syn.n_syn = E;
     dc.syn.n = n;
     dc.syn.dt_ms = cfg->dt_ms;
-    CsrScalars sc{~0ull, ~0ull, 1u, 0u};
+    CsrScalars sc{~0ull, ~0ull, 1u, ~0u, 0u};
     if (E) {
         if (!d_src) LIST_TRY(eng.pin_copy((void *)dc.syn.src, src, 4 * E));
         if (!d_tgt) LIST_TRY(eng.pin_copy((void *)dc.syn.tgt, tgt, 4 * E));
@@ -182,6 +182,7 @@ static ne2b_status create_from_list(ne2b::Engine &eng, const ne2b_net_desc *net,
                            value_at(src, d_src, j), value_at(tgt, d_tgt, j), (double)dv, (double)cfg->dt_ms));
     }
     dc.max_delay = sc.max_delay;
+    dc.min_delay = sc.min_delay;
     LIST_TRY(eng.add_net_device_csr(net, cfg, dc, slot));
     LIST_TRY(cuda_error(cudaMemcpyAsync(&sc, dc.sc, sizeof sc, cudaMemcpyDeviceToHost, st), "scatter readback"));
     LIST_TRY(cuda_error(cudaStreamSynchronize(st), "device CSR build"));
@@ -476,7 +477,7 @@ ne2b_status ne2b_set_delivery_warps(ne2b_sim *sim, int32_t on) {
 ne2b_status ne2b_delivery_warps(ne2b_sim *sim, int32_t *on, int32_t *active) {
     if (!sim || !on || !active) return set_error(NE2B_EINVAL, "null argument");
     *on = sim->eng.shape().ws ? 1 : 0;
-    *active = (!sim->eng.resident() && sim->eng.ws_applies(sim->eng.shape())) ? 1 : 0;
+    *active = (!sim->eng.resident() && !sim->eng.cluster() && sim->eng.ws_applies(sim->eng.shape())) ? 1 : 0;
     return NE2B_OK;
 }
 
@@ -742,7 +743,6 @@ ne2b_status ne2b_server_create(const ne2b_server_config *cfg, int device, ne2b_s
         s->cfg = *cfg;
         if (s->cfg.steps_per_launch == 0) s->cfg.steps_per_launch = 64;
         ne2b_status st = s->eng.init(device, cfg->int_weights != 0, cfg->max_requests);
-        if (st == NE2B_OK) st = s->eng.set_mode(ne2b::kModeStream);
         if (st == NE2B_OK) st = ne2b::cuda_error(cudaStreamCreateWithFlags(&s->rstream, cudaStreamNonBlocking), "result stream");
         for (int k = 0; k < 2 && st == NE2B_OK; ++k)
             st = ne2b::cuda_error(cudaEventCreateWithFlags(&s->step_ev[k], cudaEventDisableTiming), "event");
@@ -754,17 +754,14 @@ ne2b_status ne2b_server_create(const ne2b_server_config *cfg, int device, ne2b_s
         s->eng.fixed_grid = true;
         s->eng.multi_net = true;
         {
-            // small tiles: the most blocks per SM, so the latency chains of
+            // the streaming kernel's tiles (when a net is too large for a
+            // cluster): small ones, so the most blocks per SM, so the latency chains of
             // active tiles (state loads, scans, CSR loads) overlap; measured
             // 1.6x faster than 256x2 on the served request mix
             ne2b::TileShape sh;
             sh.block = 128;
             sh.npt = 1;
-            st = s->eng.set_shape(sh);
-            if (st != NE2B_OK) {
-                delete s;
-                return st;
-            }
+            s->eng.set_default_shape(sh);
         }
         for (uint32_t k = 0; k < std::min<uint32_t>(cfg->admission_threads, 16u); ++k) {
             auto b = std::make_unique<ne2b_server::Builder>();

@@ -59,7 +59,7 @@ __device__ __forceinline__ void st_release(uint32_t *p, uint32_t v) {
 __global__ void csr_prepass_kernel(const uint32_t *__restrict__ src, const uint32_t *__restrict__ tgt,
                                    const float *__restrict__ dly, uint64_t E, uint32_t n, float dt,
                                    uint32_t *__restrict__ counts, uint16_t *__restrict__ steps, CsrScalars *sc) {
-    uint32_t mx = 1;
+    uint32_t mx = 1, mn = ~0u;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < E; j += stride) {
         const uint32_t s = src[j], t = tgt[j];
@@ -77,10 +77,17 @@ __global__ void csr_prepass_kernel(const uint32_t *__restrict__ src, const uint3
         const uint32_t k = (uint32_t)st;
         steps[j] = (uint16_t)k;
         mx = k > mx ? k : mx;
+        mn = k < mn ? k : mn;
     }
 #pragma unroll
-    for (int o = 16; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31u) == 0u) atomicMax(&sc->max_delay, mx);
+    for (int o = 16; o; o >>= 1) {
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    }
+    if ((threadIdx.x & 31u) == 0u) {
+        atomicMax(&sc->max_delay, mx);
+        atomicMin(&sc->min_delay, mn);
+    }
 }
 
 // Block-wide exclusive sum of one value per thread (1024 threads); the

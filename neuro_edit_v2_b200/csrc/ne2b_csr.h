@@ -24,6 +24,7 @@ struct CsrScalars {
     unsigned long long bad_ref;    // first synapse with src or tgt >= n
     unsigned long long bad_delay;  // first synapse whose delay exceeds 65535 steps
     uint32_t max_delay;            // largest delay in steps (>= 1)
+    uint32_t min_delay;            // smallest delay in steps (~0 without synapses)
     uint32_t timeout;              // a scatter block gave up waiting for its predecessor
 };
 

@@ -42,10 +42,12 @@ __device__ __forceinline__ uint64_t mix64(uint64_t h) {
     return h;
 }
 
-// Poisson kick flag: state.rs:299-301, kernels.rs:128-130.
-__device__ __forceinline__ bool noise_fires(uint64_t base, float p) {
-    uint32_t h = (uint32_t)(mix64(base) >> 32);
-    return __fmul_rn(__uint2float_rn(h), 2.3283064e-10f) < p;
+// Poisson kick flag: state.rs:299-301, kernels.rs:128-130.  The reference's
+// test, f32(h) * 2.3283064e-10 < p on the hash's high half h, grows with h,
+// so it holds exactly up to the last h that the host finds for p (NetDev
+// kick_last): one integer compare instead of a conversion and a product.
+__device__ __forceinline__ bool noise_fires(uint64_t base, uint32_t kick_last) {
+    return (uint32_t)(mix64(base) >> 32) <= kick_last;
 }
 
 // Gaussian current numerator for neuron i at the step whose noise step part
@@ -57,7 +59,7 @@ __device__ __forceinline__ bool noise_fires(uint64_t base, float p) {
 // end at +-3.45 sd.  32-bit integer operations only (the 64-bit splitmix64
 // draw it replaces cost the 1M step 15% of its time), integer-exact, so CPU
 // and GPU agree bit for bit.
-__device__ __forceinline__ int32_t gauss_numer(uint32_t i, uint64_t step) {
+__device__ __forceinline__ uint32_t gauss_bytes(uint32_t i, uint64_t step) {
     uint32_t x = i ^ (uint32_t)step;
     x ^= x >> 16;
     x *= 0x7feb352du;
@@ -67,8 +69,13 @@ __device__ __forceinline__ int32_t gauss_numer(uint32_t i, uint64_t step) {
     x ^= (uint32_t)(step >> 32);
     x *= 0x9e3779b1u;
     x ^= x >> 16;
-    const uint32_t pairs = (x & 0x00ff00ffu) + ((x >> 8) & 0x00ff00ffu);  // two 16-bit byte-pair sums
-    return (int32_t)((pairs & 0xffffu) + (pairs >> 16)) - 510;
+    return x;
+}
+// Its byte sum minus 510 as a float: one byte dot product onto the bits of
+// 1.5 * 2^23, whose low mantissa bits then count whole numbers, and one exact
+// subtraction (instead of two masked adds, a fold and a conversion).
+__device__ __forceinline__ float gauss_numer(uint32_t i, uint64_t step) {
+    return __fsub_rn(__uint_as_float(__dp4a(gauss_bytes(i, step), 0x01010101u, 0x4B400000u - 510u)), 0x1.8p23f);
 }
 
 // Deterministic exp(x) for the AdEx step, in single precision: Cody-Waite

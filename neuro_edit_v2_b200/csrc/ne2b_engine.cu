@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <array>
 #include <chrono>
+#include <functional>
 #include <mutex>
 #include <thread>
 
@@ -100,6 +101,11 @@ Engine::~Engine() {
     cudaFree(d_eng_);
     cudaFree(d_block_tiles_);
     cudaFree(d_barrier_);
+    cudaFree(d_plan_);
+    for (cudaStream_t s : cl_stream_)
+        if (s) cudaStreamDestroy(s);
+    for (cudaEvent_t e : cl_ev_)
+        if (e) cudaEventDestroy(e);
     if (ev0_) cudaEventDestroy(ev0_);
     if (ev1_) cudaEventDestroy(ev1_);
     if (stream_) cudaStreamDestroy(stream_);
@@ -237,6 +243,16 @@ static float host_decay(float dt, float tau) {
 
 static void fill_noise(NetDev &d, const ne2b_config &c) {
     d.pkick = c.noise_rate_hz * c.dt_ms / 1000.0f;                 // cpu.rs:197
+    d.kick_last = 0;
+    if (d.pkick > 0.0f) {  // the last 32-bit hash h with f32(h) * 2.3283064e-10 < pkick (h = 0 always fires)
+        uint32_t lo = 0, hi = 0xffffffffu;
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo) / 2 + 1;
+            if ((float)mid * 2.3283064e-10f < d.pkick) lo = mid;
+            else hi = mid - 1;
+        }
+        d.kick_last = lo;
+    }
     d.kick = c.noise_kick_mv != 0.0f ? c.noise_kick_mv / c.dt_ms : 0.0f;  // cpu.rs:198-202
     d.gauss_k = c.gauss_sd != 0.0f ? (float)((double)c.gauss_sd * 1.7320508075688772 / 256.0) : 0.0f;
 }
@@ -418,7 +434,7 @@ ne2b_status Engine::build_net(const ne2b_net_desc *net, const ne2b_config *cfg, 
     }
     // one parallel pass over the synapses: target range, delay range, tau
     // (a device list was checked by its prepass)
-    uint32_t maxd = dc ? dc->max_delay : 1, mind = dc ? 1 : 0xffff, maxt = 0;
+    uint32_t maxd = dc ? dc->max_delay : 1, mind = dc ? dc->min_delay : 0xffff, maxt = 0;
     bool any_tau = false;
     if (!dc) {
         std::mutex mu;
@@ -692,6 +708,7 @@ ne2b_status Engine::build_net(const ne2b_net_desc *net, const ne2b_config *cfg, 
     d.seed = cfg->seed;
     d.n_inputs = net->n_inputs;
     d.rec_rows = rec_rows;
+    d.hop = std::max(1u, std::min(std::min(mind, kMaxHop), h->D - 1));  // every slot of a hop is its own
     set_step(d, 0);
     d.dt = cfg->dt_ms;
     d.decay_s = host_decay(cfg->dt_ms, cfg->synapse_tau_ms);
@@ -882,6 +899,147 @@ bool Engine::plan_resident(std::vector<Tile> &tiles, std::vector<uint32_t> &bloc
     return false;
 }
 
+// Clusters of `k`'s kind that the device holds at once (0: it does not fit):
+// those of one block of 1024 threads per SM, from the runtime the first time,
+// times the blocks that share an SM (64 registers per thread).
+int Engine::resident_clusters(const ClusterClass &k) {
+    int &one = cl_fit_[(adex_ ? 1 : 0) + (k.shape.loop ? 2 : 0) + (k.shape.one ? 4 : 0)][k.blocks];
+    if (one == 0) {
+        ClusterShape s = k.shape;
+        s.threads = kClMaxThreads;
+        // with and without the rarer features: a watch may be set later
+        one = std::min(cluster_fit(int_ring_, adex_, false, k.blocks, s, kClSmemMax),
+                       cluster_fit(int_ring_, adex_, true, k.blocks, s, kClSmemMax));
+        if (one < 1) one = -1;
+    }
+    if (one < 0 || k.smem > kClSmemMax) return 0;
+    const uint32_t per_sm = std::min<uint32_t>(kClMaxThreads / k.shape.threads, (uint32_t)(220u * 1024u / (k.smem + 4096u)));
+    return one * (int)std::max(1u, std::min(per_sm, 16u));
+}
+
+// The classes of a plan with at most `per_block` neurons per block (a net
+// takes the smallest power of two of blocks, at most 16) and `per_thread`
+// neurons per thread; returns the share of the device that they fill at
+// once, or a negative number when one does not fit.
+double Engine::cluster_classes(uint32_t per_block, uint32_t per_thread, std::vector<ClusterNet> &plan) {
+    classes_.clear();
+    plan.clear();
+    // by cluster size, kind of hop and threads (in octaves), the largest first
+    std::map<std::array<uint32_t, 3>, std::vector<const NetHost *>, std::greater<>> by;
+    for (const NetHost *h : nets_) {
+        if (!h || !h->n_pad) continue;
+        uint32_t c = 0, octave = 0;
+        while (c < 4 && ((uint64_t)per_block << c) < h->n_pad) ++c;
+        while ((32ull * per_thread << (c + octave)) < h->n_pad) ++octave;
+        by[{c, h->dev.hop > 1u ? 1u : 0u, octave}].push_back(h);
+    }
+    double filled = 0.0;
+    for (auto &e : by) {
+        ClusterClass k{};
+        k.blocks = 1u << e.first[0];
+        k.first = (uint32_t)plan.size();
+        uint32_t most = 0, hop = 1;
+        for (const NetHost *h : e.second) {
+            const uint32_t m = ((h->n_pad + k.blocks - 1) / k.blocks + 31) / 32 * 32;
+            most = std::max(most, m);
+            hop = std::max(hop, h->dev.hop);
+            plan.push_back(ClusterNet{h->slot, m});
+        }
+        k.count = (uint32_t)e.second.size();
+        k.shape.threads = std::min<uint32_t>(((most + per_thread - 1) / per_thread + 31) / 32 * 32, kClMaxThreads);
+        k.shape.loop = most > k.shape.threads;
+        k.shape.one = hop == 1u;
+        k.smem = cluster_smem(most, hop, k.shape);
+        const int fit = resident_clusters(k);
+        if (fit < 1) return -1.0;
+        filled += (double)k.count / fit;
+        classes_.push_back(k);
+    }
+    return filled;
+}
+
+// Cluster plan: each net on one cluster of 1-16 blocks; nets with the same
+// cluster size, kind of hop and threads (in octaves) share a launch.  While
+// the device holds a thread for every neuron, the nets spread over the
+// smallest blocks that all fit at once; past that, blocks of up to 2048
+// neurons with the fewest neurons per thread that fit, and past that in waves.
+// Measured, whole passes: 12 requests of 2k-43k neurons: 78 ms with blocks of
+// 256, 87 / 120 / 191 ms with blocks of 512 / 1024 / 2048; 48 liquids, 465k
+// neurons, 1500 steps: 15.1 ms with blocks of 2048 and five neurons per thread
+// (0.96 of the device), 17-20 ms with one to four (1.4-4 times the device),
+// 17-22 ms with blocks of 256 or 512.  One net alone takes a cluster up to
+// 16 x 1024 neurons: at 16,000 the step takes 0.76 us against the streaming
+// kernel's 1.84 (active: 2.5 / 3.7; AdEx 1.3 / 2.3, active 3.3 / 4.5), at
+// 24,000, in two passes, 1.8 / 1.95 (3.9 / 3.8; 2.9 / 2.5; 5.2 / 4.6).  False
+// when a tile shape or a kernel was asked for, or a net is too large or has
+// synapses with their own tau.
+bool Engine::plan_cluster(std::vector<ClusterNet> &plan) {
+    classes_.clear();
+    if (mode_ != kModeAuto || shape_set_) return false;
+    uint64_t total = 0;
+    uint32_t largest = 0;
+    for (const NetHost *h : nets_)
+        if (h) {
+            if (h->nx) return false;
+            total += h->n_pad;
+            largest = std::max(largest, h->n_pad);
+        }
+    if (!total || largest > 16u * (active_nets() > 1 ? kClMaxNeurons : kClMaxThreads)) return false;
+    for (uint32_t per_block = kClMinNeurons; per_block <= 2048u; per_block *= 2u) {
+        const double filled = cluster_classes(per_block, 1u, plan);
+        if (filled > 0.0 && filled <= 1.0) return true;
+    }
+    for (uint32_t per_thread = 2; per_thread <= 8u; ++per_thread) {
+        const double filled = cluster_classes(2048u, per_thread, plan);
+        if (filled > 0.0 && filled <= 1.0) return true;
+    }
+    return cluster_classes(2048u, 4u, plan) > 0.0;  // in waves
+}
+
+// The plan is made when steps are next run: nets may come and go in between.
+ne2b_status Engine::choose_kernel() {
+    if (!plan_stale_) return NE2B_OK;
+    std::vector<ClusterNet> plan;
+    cluster_ = !resident_ && plan_cluster(plan);
+    if (cluster_) {
+        if (!d_plan_) NE2B_CUDA(cudaMalloc(&d_plan_, sizeof(ClusterNet) * nets_cap_));
+        // pageable source, staged by the runtime before the call returns
+        NE2B_CUDA(cudaMemcpyAsync(d_plan_, plan.data(), sizeof(ClusterNet) * plan.size(), cudaMemcpyHostToDevice,
+                                  stream_));
+    }
+    plan_stale_ = false;
+    return NE2B_OK;
+}
+
+// One launch per cluster size, side by side on their own streams, forked
+// from and joined to the engine's stream.
+ne2b_status Engine::launch_clusters(uint32_t steps) {
+    bool full = false;
+    for (const NetHost *h : nets_)
+        full |= h && (h->dev.flags & (kNetRecord | kNetWatch | kNetGridWatch | kNetTraceF32));
+    const size_t nc = classes_.size();
+    while (nc > 1 && cl_ev_.size() < nc) {
+        cl_ev_.push_back(nullptr);
+        NE2B_CUDA(cudaEventCreateWithFlags(&cl_ev_.back(), cudaEventDisableTiming));
+    }
+    while (cl_stream_.size() + 1 < nc) {
+        cl_stream_.push_back(nullptr);
+        NE2B_CUDA(cudaStreamCreateWithFlags(&cl_stream_.back(), cudaStreamNonBlocking));
+    }
+    if (nc > 1) NE2B_CUDA(cudaEventRecord(cl_ev_[0], stream_));
+    for (size_t c = 0; c < nc; ++c) {
+        const ClusterClass &k = classes_[c];
+        cudaStream_t st = c == 0 ? stream_ : cl_stream_[c - 1];
+        if (c) NE2B_CUDA(cudaStreamWaitEvent(st, cl_ev_[0], 0));
+        NE2B_CUDA(launch_cluster(int_ring_, adex_, full, k.blocks, k.count, k.shape, k.smem, d_eng_,
+                                 d_plan_ + k.first, steps, st));
+        if (c) NE2B_CUDA(cudaEventRecord(cl_ev_[c], st));
+    }
+    for (size_t c = 1; c < nc; ++c) NE2B_CUDA(cudaStreamWaitEvent(stream_, cl_ev_[c], 0));
+    launches_ += nc;
+    return NE2B_OK;
+}
+
 ne2b_status Engine::rebuild_tiles() {
     const uint32_t tile = shape_.block * shape_.npt;
     std::vector<Tile> tiles;
@@ -913,6 +1071,7 @@ ne2b_status Engine::rebuild_tiles() {
     const uint32_t old_grid = grid();
     std::vector<uint32_t> block_tiles;
     resident_ = plan_resident(tiles, block_tiles);
+    plan_stale_ = true;
     if (mode_ == kModeResident && !resident_ && !tiles.empty())
         return set_error(NE2B_UNSUPPORTED, "the nets do not fit the resident kernel's shared memory");
     if (tiles.size() > tiles_cap_ || block_tiles.size() > block_tiles_cap_) NE2B_CUDA(cudaStreamSynchronize(stream_));
@@ -961,6 +1120,7 @@ ne2b_status Engine::set_shape(const TileShape &s) {
         return set_error(NE2B_EINVAL, "tile shape block=%u npt=%u is not compiled in", s.block, s.npt);
     NE2B_CUDA(cudaStreamSynchronize(stream_));
     shape_ = s;
+    shape_set_ = true;
     clear_graphs();
     return rebuild_tiles();
 }
@@ -1096,6 +1256,7 @@ ne2b_status Engine::launch_group(uint32_t steps) {
         launches_ += 2;
         return NE2B_OK;
     }
+    if (cluster_) return launch_clusters(steps);
     // the instance follows the nets' features (an external current or a
     // watch can be switched on and off between launches)
     const int var = step_variant();
@@ -1134,6 +1295,7 @@ ne2b_status Engine::launch_group(uint32_t steps) {
 
 ne2b_status Engine::run_steps(uint64_t steps) {
     NE2B_CUDA(cudaSetDevice(device_));
+    NE2B_TRY(choose_kernel());
     while (steps > 0) {
         uint64_t chunk = steps;
         for (NetHost *h : nets_)
@@ -1146,7 +1308,9 @@ ne2b_status Engine::run_steps(uint64_t steps) {
         }
         if (!repack.empty()) NE2B_TRY(pack_stim(repack));
         uint64_t left = chunk;
-        const uint64_t group = resident_ ? std::max<uint64_t>(graph_steps, resident_steps) : graph_steps;
+        const uint64_t group = cluster_    ? resident_steps
+                               : resident_ ? std::max<uint64_t>(graph_steps, resident_steps)
+                                           : graph_steps;
         while (left > 0) {
             const uint32_t g = (uint32_t)std::min<uint64_t>(left, group);
             NE2B_TRY(launch_group(g));
@@ -1494,9 +1658,37 @@ ne2b_status Engine::autotune(uint32_t steps_per_trial) {
     uint32_t blocks[32], npts[32], count = 0;
     shape_list(blocks, npts, &count);
     const int saved_mode = mode_;
+    bool best_cluster = false;
     TileShape best = shape_;
     int best_mode = mode_ == kModeAuto ? (resident_ ? kModeResident : kModeStream) : mode_;
     float best_ms = 1e30f;
+    auto trial = [&](float *ms) -> ne2b_status {
+        *ms = 1e30f;
+        NE2B_TRY(restore(snap));
+        NE2B_TRY(run_steps(graph_steps));  // capture + warm
+        for (int rep = 0; rep < 2; ++rep) {
+            NE2B_TRY(restore(snap));
+            NE2B_CUDA(cudaEventRecord(ev0_, stream_));
+            NE2B_TRY(run_steps(steps_per_trial));
+            NE2B_CUDA(cudaEventRecord(ev1_, stream_));
+            NE2B_CUDA(cudaEventSynchronize(ev1_));
+            NE2B_TRY(check_err());
+            float one = 0.0f;
+            NE2B_CUDA(cudaEventElapsedTime(&one, ev0_, ev1_));
+            *ms = std::min(*ms, one);
+        }
+        return NE2B_OK;
+    };
+    if (saved_mode == kModeAuto) {  // the cluster kernel, where it applies
+        shape_set_ = false;
+        NE2B_TRY(rebuild_tiles());
+        NE2B_TRY(choose_kernel());
+        if (cluster_) {
+            NE2B_TRY(trial(&best_ms));
+            best_cluster = true;
+        }
+    }
+    shape_set_ = true;
     for (int m : {(int)kModeStream, (int)kModeResident}) {
         if (saved_mode != kModeAuto && m != saved_mode) continue;  // a forced kernel keeps its mode
         for (uint32_t c = 0; c < 2 * count; ++c) {
@@ -1514,30 +1706,20 @@ ne2b_status Engine::autotune(uint32_t steps_per_trial) {
                 shape_ = s;
                 clear_graphs();
                 if (rebuild_tiles() != NE2B_OK) continue;  // resident plan does not fit
-                NE2B_TRY(restore(snap));
-                NE2B_TRY(run_steps(graph_steps));  // capture + warm
                 float ms = 1e30f;
-                for (int rep = 0; rep < 2; ++rep) {
-                    NE2B_TRY(restore(snap));
-                    NE2B_CUDA(cudaEventRecord(ev0_, stream_));
-                    NE2B_TRY(run_steps(steps_per_trial));
-                    NE2B_CUDA(cudaEventRecord(ev1_, stream_));
-                    NE2B_CUDA(cudaEventSynchronize(ev1_));
-                    NE2B_TRY(check_err());
-                    float one = 0.0f;
-                    NE2B_CUDA(cudaEventElapsedTime(&one, ev0_, ev1_));
-                    ms = std::min(ms, one);
-                }
+                NE2B_TRY(trial(&ms));
                 if (ms < best_ms) {
                     best_ms = ms;
+                    best_cluster = false;
                     best = s;
                     best_mode = m;
                 }
             }
         }
     }
-    mode_ = saved_mode == kModeAuto ? best_mode : saved_mode;
+    mode_ = saved_mode == kModeAuto && !best_cluster ? best_mode : saved_mode;
     shape_ = best;
+    shape_set_ = !best_cluster;
     clear_graphs();
     NE2B_TRY(rebuild_tiles());
     NE2B_TRY(restore(snap));

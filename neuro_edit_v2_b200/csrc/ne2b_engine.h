@@ -18,6 +18,7 @@
 #include "../../include/ne2b.h"
 #include "ne2b_csr.h"
 #include "ne2b_layout.h"
+#include "ne2b_step_kind.h"
 
 namespace ne2b {
 
@@ -27,7 +28,7 @@ struct DevCsrBuild {
     DevSynapses syn;
     const uint16_t *steps = nullptr;   // delay steps per list entry
     const uint32_t *counts = nullptr;  // synapses per source
-    uint32_t max_delay = 1;
+    uint32_t max_delay = 1, min_delay = ~0u;
     uint32_t *cursor = nullptr;        // [n]
     uint32_t *sums = nullptr;          // [csr_scan_blocks(n)]
     uint32_t *ticket = nullptr;        // [1], zeroed
@@ -181,6 +182,7 @@ class Engine {
     ne2b_status reset_net(uint32_t slot);
     ne2b_status sync();
     ne2b_status set_shape(const TileShape &s);
+    void set_default_shape(const TileShape &s) { shape_ = s; }  // before any net; the cluster kernel may still run
     ne2b_status autotune(uint32_t steps_per_trial);
     ne2b_status rebuild_tiles();
     ne2b_status upload_net(NetHost &h);
@@ -216,6 +218,8 @@ class Engine {
     uint64_t launches() const { return launches_; }
     void count_launches(uint64_t k) { launches_ += k; }  // kernels launched by entry points outside the engine
     bool resident() const { return resident_; }
+    // the cluster kernel runs the next steps (ne2b_cluster.cuh)
+    bool cluster() { return choose_kernel() == NE2B_OK && cluster_; }
     int mode() const { return mode_; }
     ne2b_status set_mode(int m);
     // the streaming kernel runs separate delivery warps for shape `s`
@@ -223,7 +227,7 @@ class Engine {
     bool fixed_grid = false;  // grid independent of the tile count (serving)
     bool multi_net = false;   // many nets (batch, server): the streaming kernel stages tiles ahead
     uint32_t graph_steps = 256;
-    uint32_t resident_steps = 4096;  // max steps per resident launch
+    uint32_t resident_steps = 4096;  // max steps per resident or cluster launch
     uint64_t stim_chunk = 2048;
 
   private:
@@ -237,6 +241,15 @@ class Engine {
     // the streaming kernel instance for the engine's nets (StepVariant)
     int step_variant() const;
     int step_variant(const TileShape &s) const;  // with `s`'s delivery warps where they apply
+    ne2b_status choose_kernel();
+    struct ClusterClass {  // nets with the same cluster size and kind of hop: one launch
+        uint32_t blocks, smem, first, count;
+        ClusterShape shape;
+    };
+    int resident_clusters(const ClusterClass &k);
+    double cluster_classes(uint32_t per_block, uint32_t per_thread, std::vector<ClusterNet> &plan);
+    bool plan_cluster(std::vector<ClusterNet> &plan);
+    ne2b_status launch_clusters(uint32_t steps);
     bool plan_resident(std::vector<Tile> &tiles, std::vector<uint32_t> &block_tiles);
     void clear_graphs();
 
@@ -272,6 +285,15 @@ class Engine {
     int mode_ = kModeAuto;
     bool resident_ = false;
     bool adex_ = false;  // some net holds AdEx rows: the kernels with the AdEx path run
+    // cluster kernel
+    bool cluster_ = false;
+    bool plan_stale_ = true;  // the nets or the kernel choice changed since the plan was made
+    bool shape_set_ = false;  // a tile shape was chosen: the streaming kernel runs with it
+    std::vector<ClusterClass> classes_;
+    std::map<uint32_t, int> cl_fit_[8];  // by instance, then cluster size
+    ClusterNet *d_plan_ = nullptr;
+    std::vector<cudaStream_t> cl_stream_;  // launches beside the engine's stream
+    std::vector<cudaEvent_t> cl_ev_;
     uint32_t *d_block_tiles_ = nullptr;
     uint32_t block_tiles_cap_ = 0;
     uint32_t res_neurons_ = 0;

@@ -132,6 +132,15 @@ cudaError_t launch_resident(bool int_ring, bool adex, uint32_t block, uint32_t n
     return NE2B_KIND(int_ring, adex, launch_resident(block, npt, eng, k0, nsteps, grid, smem, st));
 }
 
+int cluster_fit(bool int_ring, bool adex, bool full, uint32_t blocks, const ClusterShape &cs, size_t smem) {
+    return NE2B_KIND(int_ring, adex, cluster_fit(full, blocks, cs, smem));
+}
+
+cudaError_t launch_cluster(bool int_ring, bool adex, bool full, uint32_t blocks, uint32_t clusters,
+                           const ClusterShape &cs, size_t smem, const EngineDev *eng, const ClusterNet *plan, uint32_t steps, cudaStream_t st) {
+    return NE2B_KIND(int_ring, adex, launch_cluster(full, blocks, clusters, cs, smem, eng, plan, steps, st));
+}
+
 cudaError_t launch_barrier_selftest(unsigned int *counter, unsigned int *err, uint32_t blocks, uint32_t absent,
                                     unsigned long long limit_ns, cudaStream_t st) {
     void *args[] = {(void *)&counter, (void *)&err, (void *)&absent, (void *)&limit_ns};

@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include "ne2b_layout.h"
+#include "ne2b_step_kind.h"
 
 namespace ne2b {
 
@@ -26,6 +27,11 @@ uint32_t resident_head(uint32_t block, uint32_t npt);
 int resident_occupancy(bool int_ring, bool adex, uint32_t block, uint32_t npt, size_t smem);
 cudaError_t launch_resident(bool int_ring, bool adex, uint32_t block, uint32_t npt, const EngineDev *eng,
                             uint32_t k0, uint32_t nsteps, uint32_t grid, size_t smem, cudaStream_t st);
+// Cluster kernel (ne2b_cluster.cuh): co-resident clusters (0: it does not
+// fit), and one launch of `clusters` nets for `steps` steps, t included.
+int cluster_fit(bool int_ring, bool adex, bool full, uint32_t blocks, const ClusterShape &cs, size_t smem);
+cudaError_t launch_cluster(bool int_ring, bool adex, bool full, uint32_t blocks, uint32_t clusters,
+                           const ClusterShape &cs, size_t smem, const EngineDev *eng, const ClusterNet *plan, uint32_t steps, cudaStream_t st);
 cudaError_t launch_advance(NetDev *nets, uint32_t n_nets, uint32_t steps, cudaStream_t st);
 // Bounded grid barrier self-test: `blocks` cooperative blocks of which
 // `absent` never arrives; the others stop after `limit_ns` and set *err.

@@ -134,7 +134,12 @@ struct alignas(16) NetDev {
     // and window without a division: rphase = t % rec_rows, wphase =
     // (t + 1) % win_steps, widx0 = (t + 1) / win_steps
     uint32_t rphase, wphase, widx0;
+    uint32_t kick_last;  // pkick > 0: the largest noise hash that fires (noise_fires)
+    uint32_t hop;  // steps the cluster kernel runs between barriers: the shortest delay, at most kMaxHop
 };
+constexpr uint32_t kMaxHop = 16;
+constexpr uint32_t kClMaxNeurons = 4096;  // neurons of a cluster kernel block, at most
+constexpr uint32_t kClMinNeurons = 256;   // below this a net is not split over more blocks
 
 #ifdef __CUDACC__
 #define NE2B_HD __host__ __device__
@@ -166,6 +171,12 @@ NE2B_HD inline void set_step(NetDev &d, unsigned long long t) {
 // Mutable per-net counters, kept apart from the read-mostly descriptor.
 struct NetCounters {
     unsigned long long spikes_total;
+};
+
+// Cluster kernel: the net of one cluster and the neurons per block of it (a
+// multiple of 32).
+struct ClusterNet {
+    uint32_t net, m;
 };
 
 // Everything a step launch needs, in device memory so that a captured CUDA

@@ -160,6 +160,7 @@ __device__ __forceinline__ void process_tile(const EngineDev *__restrict__ eng, 
     const size_t slot_off = (size_t)tmod * n_pad;
     const float dt = nd.dt, decay_s = nd.decay_s;
     const float pkick = nd.pkick, kick = nd.kick, gauss_k = nd.gauss_k;
+    const uint32_t kick_last = nd.kick_last;
     const uint64_t nbase = nd.noise_step + (uint64_t)k * kNoiseStepMul;  // = noise_base_step(t, seed)
     const uint32_t tlast = nd.trace_last;
     uint32_t *__restrict__ ringw = (uint32_t *)nd.ring;
@@ -280,9 +281,9 @@ __device__ __forceinline__ void process_tile(const EngineDev *__restrict__ eng, 
             p[8] = p2.x; p[9] = p2.y;
         }
         const float gain = (ADEX && adex) ? p[0] : 1.0f;  // model/mod.rs:104-106, adex.rs:189-191
-        if (pkick > 0.0f && noise_fires(noise_base_at(i, nbase), pkick)) I = __fadd_rn(I, __fmul_rn(kick, gain));
+        if (pkick > 0.0f && noise_fires(noise_base_at(i, nbase), kick_last)) I = __fadd_rn(I, __fmul_rn(kick, gain));
         if (gauss_k != 0.0f)
-            I = __fadd_rn(I, __fmul_rn(__int2float_rn(gauss_numer(i, nbase)), __fmul_rn(gauss_k, gain)));
+            I = __fadd_rn(I, __fmul_rn(gauss_numer(i, nbase), __fmul_rn(gauss_k, gain)));
         bool sp;
         if (ADEX && adex) sp = adex_step(p, v[q], u[q], I, dt);
         else sp = izh_step(p, v[q], u[q], I, dt);
@@ -926,7 +927,66 @@ __global__ void __launch_bounds__(BLOCK) resident_kernel(const EngineDev *__rest
     }
 }
 
+}  // namespace ne2b
+#include "ne2b_cluster.cuh"
+namespace ne2b {
+
 // ------------------------------------------------ per-kind launchers
+// The launch configuration of a cluster kernel; `attr` holds one entry.
+static inline cudaLaunchConfig_t cluster_config(uint32_t blocks, uint32_t clusters, uint32_t threads, size_t smem,
+                                                cudaStream_t st, cudaLaunchAttribute *attr) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks * clusters);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = blocks;
+    attr->val.clusterDim.y = 1;
+    attr->val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+template <bool INT, bool ADEX, bool FULL, bool ONE>
+static auto cluster_instance(const ClusterShape &cs) {
+    return cs.loop ? cluster_kernel<INT, ADEX, FULL, true, ONE> : cluster_kernel<INT, ADEX, FULL, false, ONE>;
+}
+template <bool INT, bool ADEX>
+static auto cluster_instance(bool full, const ClusterShape &cs) {
+    return full ? (cs.one ? cluster_instance<INT, ADEX, true, true>(cs) : cluster_instance<INT, ADEX, true, false>(cs))
+                : (cs.one ? cluster_instance<INT, ADEX, false, true>(cs)
+                          : cluster_instance<INT, ADEX, false, false>(cs));
+}
+
+template <bool INT, bool ADEX>
+int StepKind<INT, ADEX>::cluster_fit(bool full, uint32_t blocks, const ClusterShape &cs, size_t smem) {
+    auto *k = cluster_instance<INT, ADEX>(full, cs);
+    if (smem > kClSmemMax ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClSmemMax) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+        return 0;
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = cluster_config(blocks, 1, cs.threads, smem, nullptr, attr);
+    int c = 0;
+    if (cudaOccupancyMaxActiveClusters(&c, k, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return c;
+}
+
+template <bool INT, bool ADEX>
+cudaError_t StepKind<INT, ADEX>::launch_cluster(bool full, uint32_t blocks, uint32_t clusters,
+                                                const ClusterShape &cs, size_t smem, const EngineDev *eng,
+                                                const ClusterNet *plan, uint32_t steps, cudaStream_t st) {
+    auto *k = cluster_instance<INT, ADEX>(full, cs);
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = cluster_config(blocks, clusters, cs.threads, smem, st, attr);
+    return cudaLaunchKernelEx(&cfg, k, eng, plan, steps);
+}
+
 template <typename... Args>
 static cudaError_t launch_pdl(void (*kernel)(Args...), uint32_t grid, uint32_t block, cudaStream_t st, bool pdl,
                               Args... args) {

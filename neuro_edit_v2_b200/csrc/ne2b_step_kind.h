@@ -43,8 +43,29 @@ enum StepVariant : int { kStepSingle = 0, kStepMulti = 1, kStepPlain = 2, kStepM
 // (separate delivery warps; engines of one net, NE2B_WS_SHAPES only).
 constexpr int kStepWS = 0x10;
 
+constexpr size_t kClSmemMax = 200 * 1024;  // dynamic shared memory of a cluster kernel block, at most
+constexpr uint32_t kClMaxThreads = 1024;  // threads of a cluster kernel block, at most
+
+// A cluster kernel block: threads, whether its range takes several passes of
+// them (state in shared memory), and whether every hop is 1.
+struct ClusterShape {
+    uint32_t threads;
+    bool loop, one;
+};
+// Its shared memory: the hop's spike counters and lists (u16 per neuron and
+// step), then (loop) the state (16 bytes per neuron).
+inline uint32_t cluster_smem(uint32_t m, uint32_t hop, const ClusterShape &s) {
+    return (s.one ? 0u : kMaxHop * 4u + m * hop * 2u) + (s.loop ? m * 16u : 0u);
+}
+
 template <bool INT, bool ADEX>
 struct StepKind {
+    // cluster kernel: `clusters` clusters of `blocks` blocks; `full` = with
+    // records, custom-tau synapses, f32 trace and watches
+    static int cluster_fit(bool full, uint32_t blocks, const ClusterShape &cs, size_t smem);
+    static cudaError_t launch_cluster(bool full, uint32_t blocks, uint32_t clusters, const ClusterShape &cs,
+                                      size_t smem, const EngineDev *eng, const ClusterNet *plan, uint32_t steps,
+                                      cudaStream_t st);
     static int occupancy(uint32_t block, uint32_t npt, int variant);
     static cudaError_t launch(uint32_t block, uint32_t npt, int variant, const EngineDev *eng, uint32_t k_step,
                               uint32_t grid, cudaStream_t st);

@@ -7,24 +7,26 @@
 // fit_ridge_multi:
 //   1. column means mu (f64, rows summed in order) and the centred design
 //      Xc = x - mu (f64);
-//   2. the Gram matrix G = Xc Xc^T + lambda I: tiled in shared memory, each
-//      thread owning 2 x 2 entries and summing each dot product exactly as
+//   2. the Gram matrix G = Xc Xc^T + lambda I, each entry summed exactly as
 //      the reference does (four accumulators by column mod 4, the tail
 //      apart, then tail + ((a0 + a1) + a2) + a3);
-//   3. Cholesky G = L L^T in place, right-looking: column j is divided by
-//      sqrt(G[j][j]), then the trailing lower triangle loses
-//      L[i][j] L[k][j] — every entry meets its subtractions in the same
-//      order k = 0, 1, ... as the reference's left-looking loop;
-//   4. per class, L z = y and L^T a = z on the host (T^2 work), in the
-//      reference's loop order;
+//   3. Cholesky G = U^T U in place of the upper triangle, in panels of 32
+//      rows: every entry meets its subtractions in the same order k = 0, 1,
+//      ... as the reference's left-looking loop;
+//   4. U^T z = y and U a = z per class on the host (T^2 work).  The second
+//      sums ascend from the entry computed last, as the reference's do, so
+//      each class is one chain of T^2 / 2 dependent subtractions, which a
+//      CPU core runs three times faster than a GPU thread; four classes go
+//      side by side;
 //   5. w = Xc^T a on the device (rows summed in order), bias on the host.
 //
-// fit_ridge: the (F + 1) x (F + 1) normal matrix, each entry summed over the
-// rows in order as the reference accumulates it, the bias column, lambda on
-// the diagonal and off the bias again ((s + lambda) - lambda, as there), the
-// same Cholesky, and the solve on the host; a matrix that is not positive
-// definite is refactored with 1e-3 + lambda more on the diagonal (from a
-// copy kept on the device), then gives zeros.
+// fit_ridge: the normal matrix of [X 1 y], each entry summed over the rows
+// in order as the reference accumulates it (the products with 1 are exact,
+// so the bias column and the right-hand side are sums of the same kind),
+// lambda on the diagonal and off the bias again ((s + lambda) - lambda, as
+// there), the same Cholesky, and the solve on the host; a matrix that is not
+// positive definite is refactored with 1e-3 + lambda more on the diagonal
+// (from a copy kept on the device), then gives zeros.
 //
 // Every f64 operation is an explicit round-to-nearest intrinsic, so nothing
 // is contracted into an FMA: the weights equal the reference's bit for bit.
@@ -32,10 +34,14 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <algorithm>
+#include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "ne2b_engine.h"
 #include "ne2b_handles.h"
+#include "ne2b_solve.h"
 
 #define NE2B_CUDA(call)                                      \
     do {                                                     \
@@ -51,15 +57,74 @@
 namespace ne2b {
 namespace {
 
-constexpr uint32_t kGramTile = 32;  // 32 x 32 Gram entries per block, 16 x 16 threads
-constexpr uint32_t kGramK = 32;     // columns staged per pass (a multiple of 4)
+constexpr uint32_t kTile = 32;    // 32 x 32 entries per block, 8 x 8 threads of 4 x 4
+constexpr uint32_t kChunk = 32;   // terms staged per pass (a multiple of 4)
+constexpr uint32_t kPitch = kTile + 2;  // doubles per staged term: rows stay 16-byte aligned
+constexpr uint32_t kPanel = 32;   // Cholesky rows per panel
+constexpr uint32_t kUpdTile = 64; // trailing update: 64 x 64 entries per block, 16 x 16 threads of 4 x 4
 
-__global__ void col_mean_kernel(const float *__restrict__ x, uint32_t t, uint32_t f, double *__restrict__ mu) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= f) return;
+// linear block id -> (bi, bj), bi <= bj
+__device__ __forceinline__ void triangle_tile(uint32_t id, uint32_t &bi, uint32_t &bj) {
+    bj = (uint32_t)((sqrt(8.0 * id + 1.0) - 1.0) / 2.0);
+    while ((bj + 1) * (bj + 2) / 2 <= id) ++bj;
+    while (bj * (bj + 1) / 2 > id) --bj;
+    bi = id - bj * (bj + 1) / 2;
+}
+
+// A thread's four rows (or columns) of a W-wide tile: 2 k, 2 k + 1, W / 2 + 2 k
+// and W / 2 + 2 k + 1, so that neighbouring threads' 16-byte loads are neighbours in
+// shared memory (four consecutive ones would collide on every other bank).
+template <uint32_t W>
+__device__ __forceinline__ uint32_t spread4(uint32_t k, uint32_t e) { return (e >> 1) * (W / 2u) + 2u * k + (e & 1u); }
+template <uint32_t W>
+__device__ __forceinline__ void load_spread4(const double *row, uint32_t k, double (&v)[4]) {  // row 16-byte aligned
+    const double2 a = *reinterpret_cast<const double2 *>(row + 2u * k);
+    const double2 b = *reinterpret_cast<const double2 *>(row + W / 2u + 2u * k);
+    v[0] = a.x;
+    v[1] = a.y;
+    v[2] = b.x;
+    v[3] = b.y;
+}
+__device__ __forceinline__ void load4(const double *p, double (&v)[4]) {  // p 16-byte aligned
+    const double2 a = *reinterpret_cast<const double2 *>(p), b = *reinterpret_cast<const double2 *>(p + 2);
+    v[0] = a.x;
+    v[1] = a.y;
+    v[2] = b.x;
+    v[3] = b.y;
+}
+
+// 32 columns per block: all four warps stage 128 rows while the first adds
+// the 128 before them in order (24 us at 1000 x 4320; T serial loads by F
+// threads took 66 us).
+__global__ void __launch_bounds__(128) col_mean_kernel(const float *__restrict__ x, uint32_t t, uint32_t f,
+                                                       double *__restrict__ mu) {
+    constexpr uint32_t R = 128;
+    __shared__ float sx[2][R][32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t c = blockIdx.x * 32u + lane;
+    auto stage = [&](uint32_t r0, uint32_t buf) {
+        float v[R / 4u];
+#pragma unroll
+        for (uint32_t e = 0; e < R / 4u; ++e) {
+            const uint32_t r = r0 + 4u * e + warp;
+            v[e] = r < t && c < f ? x[(size_t)r * f + c] : 0.0f;
+        }
+#pragma unroll
+        for (uint32_t e = 0; e < R / 4u; ++e) sx[buf][4u * e + warp][lane] = v[e];
+    };
     double s = 0.0;
-    for (uint32_t r = 0; r < t; ++r) s = __dadd_rn(s, (double)x[(size_t)r * f + c]);
-    mu[c] = __ddiv_rn(s, (double)t);
+    stage(0u, 0u);
+    __syncthreads();
+    for (uint32_t r0 = 0, buf = 0; r0 < t; r0 += R, buf ^= 1u) {
+        if (warp == 0u) {
+            const uint32_t rn = min(R, t - r0);
+#pragma unroll 8
+            for (uint32_t r = 0; r < rn; ++r) s = __dadd_rn(s, (double)sx[buf][r][lane]);
+        }
+        if (r0 + R < t) stage(r0 + R, buf ^ 1u);
+        __syncthreads();
+    }
+    if (warp == 0u && c < f) mu[c] = __ddiv_rn(s, (double)t);
 }
 
 __global__ void center_kernel(const float *__restrict__ x, uint64_t n, uint32_t f, const double *__restrict__ mu,
@@ -68,170 +133,284 @@ __global__ void center_kernel(const float *__restrict__ x, uint64_t n, uint32_t 
         xc[i] = __dsub_rn((double)x[i], mu[i % f]);
 }
 
-// Lower-triangle tiles (bi >= bj) of G = Xc Xc^T; the diagonal gets lambda;
-// both halves are written.
-__global__ void __launch_bounds__(256) gram_kernel(const double *__restrict__ xc, uint32_t t, uint32_t f,
-                                                   double lambda, double *__restrict__ g) {
-    __shared__ double sa[kGramTile][kGramK + 1];
-    __shared__ double sb[kGramTile][kGramK + 1];
-    // linear block id -> (bi, bj), bj <= bi
-    const uint32_t id = blockIdx.x;
-    uint32_t bi = (uint32_t)((sqrt(8.0 * id + 1.0) - 1.0) / 2.0);
-    while ((bi + 1) * (bi + 2) / 2 <= id) ++bi;
-    while (bi * (bi + 1) / 2 > id) --bi;
-    const uint32_t bj = id - bi * (bi + 1) / 2;
-    const uint32_t i0 = bi * kGramTile, j0 = bj * kGramTile;
-    const uint32_t tx = threadIdx.x & 15u, ty = threadIdx.x >> 4;
-    double acc[2][2][4] = {};
-    double tail[2][2] = {};
+__device__ __forceinline__ void copy_async8(double *smem, const double *g) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(g)
+                 : "memory");
+}
+
+__device__ __forceinline__ void copy_async16(double *smem, const double *g) {  // both 16-byte aligned
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(g)
+                 : "memory");
+}
+
+// Upper-triangle tiles of G = Xc Xc^T; the diagonal gets lambda.  Bound by
+// the f64 pipe (T^2 F multiplies and adds, never fused): each thread owns
+// 4 x 4 entries, so one column's 8 operands from shared memory feed 32
+// operations, and the next 32 columns arrive by cp.async meanwhile.  Blocks
+// of two warps keep the tiles small: 528 of them at T = 1000, spread evenly.
+// Measured at 1000 x 4320: 457 us, 9.4e12
+// operations per second (2 x 2 entries per thread, 256 threads: 1076 us).
+__global__ void __launch_bounds__(64) gram_kernel(const double *__restrict__ xc, uint32_t t, uint32_t f,
+                                                  double lambda, double *__restrict__ g) {
+    __shared__ __align__(16) double sa[2][kChunk][kPitch], sb[2][kChunk][kPitch];
+    uint32_t bi, bj;
+    triangle_tile(blockIdx.x, bi, bj);
+    const uint32_t i0 = bi * kTile, j0 = bj * kTile;
+    const uint32_t tx = threadIdx.x & 7u, ty = threadIdx.x >> 3, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t f4 = f / 4u * 4u;
-    for (uint32_t k0 = 0; k0 < f; k0 += kGramK) {
-        for (uint32_t e = threadIdx.x; e < kGramTile * kGramK; e += 256) {
-            const uint32_t r = e / kGramK, c = e % kGramK;
-            const bool in_c = k0 + c < f;
-            sa[r][c] = (i0 + r < t && in_c) ? xc[(size_t)(i0 + r) * f + k0 + c] : 0.0;
-            sb[r][c] = (j0 + r < t && in_c) ? xc[(size_t)(j0 + r) * f + k0 + c] : 0.0;
-        }
+    auto stage = [&](uint32_t k0, uint32_t buf) {
+        if (k0 + lane < f4)
+            for (uint32_t r = warp; r < kTile; r += 2u) {
+                copy_async8(&sa[buf][lane][r], xc + (size_t)min(i0 + r, t - 1u) * f + k0 + lane);
+                copy_async8(&sb[buf][lane][r], xc + (size_t)min(j0 + r, t - 1u) * f + k0 + lane);
+            }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double acc[4][4][4] = {};
+    stage(0u, 0u);
+    for (uint32_t k0 = 0, buf = 0; k0 < f4; k0 += kChunk, buf ^= 1u) {
+        stage(k0 + kChunk, buf ^ 1u);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
-        const uint32_t kn = min(kGramK, f - k0);
-        uint32_t c = 0;
-        // k0 and f4 are multiples of 4: whole groups of four below f4, each
-        // column into its accumulator (static indices keep them in registers)
-        for (; c + 4u <= kn && k0 + c + 4u <= f4; c += 4u)
+        const uint32_t kn = min(kChunk, f4 - k0);
+        for (uint32_t c = 0; c < kn; c += 4u)
 #pragma unroll
-            for (int a = 0; a < 2; ++a)
+            for (int q = 0; q < 4; ++q) {
+                double av[4], bv[4];
+                load_spread4<kTile>(sa[buf][c + q], ty, av);
+                load_spread4<kTile>(sb[buf][c + q], tx, bv);
 #pragma unroll
-                for (int b = 0; b < 2; ++b)
+                for (int a = 0; a < 4; ++a)
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        acc[a][b][q] = __dadd_rn(acc[a][b][q], __dmul_rn(sa[ty * 2 + a][c + q], sb[tx * 2 + b][c + q]));
-        for (; c < kn; ++c)  // the columns from f4 on
-#pragma unroll
-            for (int a = 0; a < 2; ++a)
-#pragma unroll
-                for (int b = 0; b < 2; ++b)
-                    tail[a][b] = __dadd_rn(tail[a][b], __dmul_rn(sa[ty * 2 + a][c], sb[tx * 2 + b][c]));
+                    for (int b = 0; b < 4; ++b) acc[a][b][q] = __dadd_rn(acc[a][b][q], __dmul_rn(av[a], bv[b]));
+            }
         __syncthreads();
     }
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            const uint32_t i = i0 + ty * 2 + a, j = j0 + tx * 2 + b;
-            if (i >= t || j >= t || j > i) continue;
+        for (int b = 0; b < 4; ++b) {
+            const uint32_t i = i0 + spread4<kTile>(ty, a), j = j0 + spread4<kTile>(tx, b);
+            if (i >= t || j >= t || j < i) continue;
+            double tail = 0.0;
+            for (uint32_t c = f4; c < f; ++c)
+                tail = __dadd_rn(tail, __dmul_rn(xc[(size_t)j * f + c], xc[(size_t)i * f + c]));
             const double *q = acc[a][b];
-            double s = __dadd_rn(tail[a][b], __dadd_rn(__dadd_rn(__dadd_rn(q[0], q[1]), q[2]), q[3]));
+            double s = __dadd_rn(tail, __dadd_rn(__dadd_rn(__dadd_rn(q[0], q[1]), q[2]), q[3]));
             if (i == j) s = __dadd_rn(s, lambda);
             g[(size_t)i * t + j] = s;
-            g[(size_t)j * t + i] = s;
         }
 }
 
-// Column j below the diagonal divided by sqrt(G[j][j]); a non-positive
-// pivot raises *bad (the matrix is not positive definite).
-__global__ void chol_column_kernel(double *g, uint32_t t, uint32_t j, unsigned int *bad) {
-    const double d = g[(size_t)j * t + j];
-    if (d <= 0.0) {  // the reference's test (readout.rs:155): a NaN pivot carries on
-        if (blockIdx.x == 0 && threadIdx.x == 0) atomicExch(bad, 1u);
-        return;
+// Rows [p, p + kPanel) of U.  Warp 0 of every block factors the panel's
+// diagonal block (lane i holds column i) while the other warps' threads
+// divide and update one column to the right of it each, a row behind: they
+// take row j - 1 from shared memory as warp 0 works on row j.  A latency
+// chain of 32 square roots and divisions; in the place of two launches per
+// row it serves 32 rows at once: 15.5 us a panel at 1000 rows, with the
+// update 0.82 ms in all, against 7.8 ms.  The loop over j is rolled (the registers
+// move up one place per j) so that a launch's code, which runs once, is
+// short.  The factored diagonal block goes to dblk, because other blocks may
+// still be reading the original; the trailing update puts it in place (the
+// last panel, one block, does so itself).  A non-positive pivot raises *bad
+// (the matrix is not positive definite).
+constexpr uint32_t kPanelCols = 96;  // columns right of the panel per block
+__global__ void __launch_bounds__(32 + kPanelCols) chol_panel_kernel(double *g, uint32_t n, uint32_t p,
+                                                                     double *__restrict__ dblk, unsigned int *bad) {
+    __shared__ double sd[kPanel][2u * kPanel];  // sd[j][k] = U[p + j][p + k], k >= j; read up to k = j + 31
+    if (*bad) return;  // set by an earlier panel: uniform
+    const uint32_t nb = min(kPanel, n - p), lane = threadIdx.x & 31u;
+    const bool diag = threadIdx.x < 32u;
+    // columns to the right exist only past a full panel
+    const uint32_t i = diag ? p + lane : p + kPanel + blockIdx.x * kPanelCols + threadIdx.x - 32u;
+    const bool active = diag ? lane < nb : i < n;
+    double c[kPanel];  // c[k]: row j + k of column i
+#pragma unroll
+    for (uint32_t j = 0; j < kPanel; ++j) {
+        c[j] = active && j < nb && p + j <= i ? g[(size_t)(p + j) * n + i] : 1.0;
+        if (diag) sd[j][kPanel + lane] = 0.0;
     }
-    const double ljj = __dsqrt_rn(d);
-    const uint32_t i = j + 1u + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < t) g[(size_t)i * t + j] = __ddiv_rn(g[(size_t)i * t + j], ljj);
+    bool stop = false;
+#pragma unroll 1
+    for (uint32_t s = 0; s <= kPanel; ++s) {
+        const uint32_t j = diag ? s : s - 1u;  // this warp's row
+        if (j < kPanel) {
+            double l;
+            if (diag) {
+                const double d = __shfl_sync(0xffffffffu, c[0], j);
+                stop |= j < nb && d <= 0.0;  // the reference's test (readout.rs:155): a NaN pivot carries on
+                const double ljj = __dsqrt_rn(d);
+                l = lane == j ? ljj : __ddiv_rn(c[0], ljj);
+                sd[j][lane] = l;
+                __syncwarp();
+            } else {
+                l = __ddiv_rn(c[0], sd[j][j]);
+            }
+            if (!diag) {
+                if (active) g[(size_t)(p + j) * n + i] = l;
+            } else if (blockIdx.x == 0u && active && j < nb && lane >= j) {
+                if (p + kPanel < n) dblk[j * kPanel + lane] = l;
+                else g[(size_t)(p + j) * n + i] = l;
+            }
+#pragma unroll
+            for (uint32_t k = 1; k < kPanel; ++k)  // row j + k loses U[j][j + k] U[j][i]
+                c[k - 1] = __dsub_rn(c[k], __dmul_rn(l, sd[j][j + k]));
+        }
+        __syncthreads();
+    }
+    if (stop && blockIdx.x == 0u && lane == 0u) atomicExch(bad, 1u);
 }
 
-// G[i][k] -= L[i][j] L[k][j] for j < k <= i; G[j][j] becomes sqrt(G[j][j]).
-__global__ void chol_update_kernel(double *g, uint32_t t, uint32_t j, const unsigned int *bad) {
+// The trailing upper triangle past a full panel: G[k][i] -= U[p + j][k]
+// U[p + j][i] for j = 0..31 in order, from registers (one read and one write
+// of the matrix per 32 rows).
+__global__ void __launch_bounds__(256) chol_update_kernel(double *g, uint32_t n, uint32_t p,
+                                                          const double *__restrict__ dblk, const unsigned int *bad) {
+    __shared__ __align__(16) double sk[kPanel][kUpdTile], si[kPanel][kUpdTile];
     if (*bad) return;
-    const uint32_t k = j + 1u + blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t i = j + 1u + blockIdx.y * blockDim.y + threadIdx.y;
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0)
-        g[(size_t)j * t + j] = __dsqrt_rn(g[(size_t)j * t + j]);
-    if (i >= t || k > i) return;
-    g[(size_t)i * t + k] = __dsub_rn(g[(size_t)i * t + k], __dmul_rn(g[(size_t)i * t + j], g[(size_t)k * t + j]));
-}
-
-// w[c][q] = sum over rows r (in order) of a[c][r] xc[r][q].
-__global__ void weights_kernel(const double *__restrict__ xc, const double *__restrict__ a, uint32_t t, uint32_t f,
-                               uint32_t k, double *__restrict__ w) {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t c = blockIdx.y;
-    if (q >= f) return;
-    double s = 0.0;
-    for (uint32_t r = 0; r < t; ++r) s = __dadd_rn(s, __dmul_rn(a[(size_t)c * t + r], xc[(size_t)r * f + q]));
-    w[(size_t)c * f + q] = s;
-}
-
-// Upper-triangle tiles (bi <= bj) of the normal matrix: a[i][j] = sum over
-// rows r, in order, of x[r][i] x[r][j] (f32 read as f64); both halves of
-// the (F + 1)-wide matrix are written.
-__global__ void __launch_bounds__(256) normal_kernel(const float *__restrict__ x, uint32_t t, uint32_t f,
-                                                     double *__restrict__ a) {
-    __shared__ double si[kGramK][kGramTile + 1];
-    __shared__ double sj[kGramK][kGramTile + 1];
-    const uint32_t id = blockIdx.x;
-    uint32_t bj = (uint32_t)((sqrt(8.0 * id + 1.0) - 1.0) / 2.0);
-    while ((bj + 1) * (bj + 2) / 2 <= id) ++bj;
-    while (bj * (bj + 1) / 2 > id) --bj;
-    const uint32_t bi = id - bj * (bj + 1) / 2;  // bi <= bj
-    const uint32_t i0 = bi * kGramTile, j0 = bj * kGramTile, nf = f + 1u;
+    if (blockIdx.x == 0u)  // the panel's diagonal block, which nothing here reads
+        for (uint32_t e = threadIdx.x; e < kPanel * kPanel; e += 256u)
+            if (e % kPanel >= e / kPanel) g[(size_t)(p + e / kPanel) * n + p + e % kPanel] = dblk[e];
+    uint32_t bk, bi;
+    triangle_tile(blockIdx.x, bk, bi);
+    const uint32_t q0 = p + kPanel, k0 = q0 + bk * kUpdTile, i0 = q0 + bi * kUpdTile;
+    for (uint32_t e = threadIdx.x; e < kPanel * kUpdTile; e += 256u) {
+        const uint32_t j = e / kUpdTile, c = e % kUpdTile;
+        sk[j][c] = g[(size_t)(p + j) * n + min(k0 + c, n - 1u)];
+        si[j][c] = g[(size_t)(p + j) * n + min(i0 + c, n - 1u)];
+    }
     const uint32_t tx = threadIdx.x & 15u, ty = threadIdx.x >> 4;
-    double acc[2][2] = {};
-    for (uint32_t r0 = 0; r0 < t; r0 += kGramK) {
-        for (uint32_t e = threadIdx.x; e < kGramK * kGramTile; e += 256) {
-            const uint32_t r = e / kGramTile, c = e % kGramTile;
-            const bool in_r = r0 + r < t;
-            si[r][c] = (in_r && i0 + c < f) ? (double)x[(size_t)(r0 + r) * f + i0 + c] : 0.0;
-            sj[r][c] = (in_r && j0 + c < f) ? (double)x[(size_t)(r0 + r) * f + j0 + c] : 0.0;
+    double acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const uint32_t k = k0 + spread4<kUpdTile>(ty, a), i = i0 + spread4<kUpdTile>(tx, b);
+            acc[a][b] = k < n && i < n ? g[(size_t)k * n + i] : 0.0;
         }
-        __syncthreads();
-        const uint32_t rn = min(kGramK, t - r0);
-        for (uint32_t r = 0; r < rn; ++r)
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t j = 0; j < kPanel; ++j) {
+        double kv[4], iv[4];
+        load_spread4<kUpdTile>(sk[j], ty, kv);
+        load_spread4<kUpdTile>(si[j], tx, iv);
 #pragma unroll
-            for (int p = 0; p < 2; ++p)
+        for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int q = 0; q < 2; ++q)
-                    acc[p][q] = __dadd_rn(acc[p][q], __dmul_rn(si[r][ty * 2 + p], sj[r][tx * 2 + q]));
-        __syncthreads();
+            for (int b = 0; b < 4; ++b) acc[a][b] = __dsub_rn(acc[a][b], __dmul_rn(iv[b], kv[a]));
     }
 #pragma unroll
-    for (int p = 0; p < 2; ++p)
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const uint32_t i = i0 + ty * 2 + p, j = j0 + tx * 2 + q;
-            if (i >= f || j >= f || i > j) continue;
-            a[(size_t)i * nf + j] = acc[p][q];
-            a[(size_t)j * nf + i] = acc[p][q];
+        for (int b = 0; b < 4; ++b) {
+            const uint32_t k = k0 + spread4<kUpdTile>(ty, a), i = i0 + spread4<kUpdTile>(tx, b);
+            if (k < n && i < n && k <= i) g[(size_t)k * n + i] = acc[a][b];
         }
 }
 
-// The bias column (sum of each feature over the rows, in order), the
-// right-hand side b[i] = sum of x[r][i] y[r], and b[f] = sum of y.
-__global__ void bias_rhs_kernel(const float *__restrict__ x, const float *__restrict__ y, uint32_t t, uint32_t f,
-                                double *__restrict__ a, double *__restrict__ b) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t nf = f + 1u;
-    if (j > f) return;
-    double s = 0.0, sb = 0.0;
-    for (uint32_t r = 0; r < t; ++r) {
-        const double yr = (double)y[r];
-        if (j < f) {
-            const double xv = (double)x[(size_t)r * f + j];
-            s = __dadd_rn(s, xv);
-            sb = __dadd_rn(sb, __dmul_rn(xv, yr));
-        } else {
-            sb = __dadd_rn(sb, yr);
+// w[c][q] = sum over rows r (in order) of a[c][r] xc[r][q]: a thread takes
+// one column for four classes, the next 16 rows' loads in flight while this
+// 16 are added, the dual weights broadcast from shared memory (74 us for 4
+// classes at 1000 x 4320; a thread per column and class: 122 us).
+__global__ void __launch_bounds__(32) weights_kernel(const double *__restrict__ xc, const double *__restrict__ a,
+                                                     uint32_t t, uint32_t f, uint32_t k, double *__restrict__ w) {
+    constexpr uint32_t R = 16;
+    __shared__ __align__(16) double sa[R][4];
+    const uint32_t q = blockIdx.x * 32u + threadIdx.x, c0 = blockIdx.y * 4u, qq = min(q, f - 1u);
+    double v[R], nx[R], av[2], s[4] = {};
+    // two of the 16 x 4 dual weights per thread: row lane / 2, classes 2 (lane % 2) and the next
+    const uint32_t ar = threadIdx.x >> 1, ac = (threadIdx.x & 1u) * 2u;
+    auto fetch = [&](uint32_t r0, double (&d)[R]) {
+#pragma unroll
+        for (uint32_t e = 0; e < R; ++e) d[e] = r0 + e < t ? xc[(size_t)(r0 + e) * f + qq] : 0.0;
+#pragma unroll
+        for (uint32_t e = 0; e < 2u; ++e)
+            av[e] = r0 + ar < t ? a[(size_t)min(c0 + ac + e, k - 1u) * t + r0 + ar] : 0.0;
+    };
+    fetch(0u, v);
+    for (uint32_t r0 = 0; r0 < t; r0 += R) {
+        sa[ar][ac] = av[0];
+        sa[ar][ac + 1u] = av[1];
+        __syncwarp();
+        fetch(r0 + R, nx);
+#pragma unroll
+        for (uint32_t e = 0; e < R; ++e) {
+            double a4[4];
+            load4(sa[e], a4);
+            if (r0 + e < t)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) s[c] = __dadd_rn(s[c], __dmul_rn(a4[c], v[e]));
+            v[e] = nx[e];
         }
+        __syncwarp();
     }
-    b[j] = sb;
-    if (j < f) {
-        a[(size_t)j * nf + f] = s;
-        a[(size_t)f * nf + j] = s;
-    } else {
-        double ones = 0.0;
-        for (uint32_t r = 0; r < t; ++r) ones = __dadd_rn(ones, 1.0);
-        a[(size_t)f * nf + f] = ones;
+#pragma unroll
+    for (uint32_t c = 0; c < 4u; ++c)
+        if (q < f && c0 + c < k) w[(size_t)(c0 + c) * f + q] = s[c];
+}
+
+// The columns [x 1 y] as f64, rows of `pitch` doubles (even: 16-byte aligned;
+// zeros past y).
+__global__ void augment_kernel(const float *__restrict__ x, const float *__restrict__ y, uint32_t t, uint32_t f,
+                               uint32_t pitch, double *__restrict__ xa) {
+    const uint32_t r = blockIdx.y;
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < pitch; c += gridDim.x * blockDim.x)
+        xa[(size_t)r * pitch + c] = c < f ? (double)x[(size_t)r * f + c] : c == f ? 1.0 : c == f + 1u ? (double)y[r] : 0.0;
+}
+
+// Upper-triangle tiles of the normal matrix of the columns [x 1 y], each
+// entry summed over the rows in order: a (F + 1 wide) and, from the last
+// column, the right-hand side.  4 x 4 entries per thread and cp.async as in
+// gram_kernel; the conversion to f64 is done once beforehand (on the way to
+// shared memory it took as long as the sums).  166 us at 1200 x 1080 with the
+// conversion, against 249 + 315 us with 2 x 2 entries per thread and a thread
+// per column for the bias and right-hand side.
+__global__ void __launch_bounds__(64) normal_kernel(const double *__restrict__ xa, uint32_t t, uint32_t f,
+                                                    uint32_t pitch, double *__restrict__ a,
+                                                    double *__restrict__ rhs) {
+    __shared__ __align__(16) double si[2][kChunk][kTile], sj[2][kChunk][kTile];
+    uint32_t bi, bj;
+    triangle_tile(blockIdx.x, bi, bj);
+    const uint32_t i0 = bi * kTile, j0 = bj * kTile, nf = f + 1u;
+    const uint32_t tx = threadIdx.x & 7u, ty = threadIdx.x >> 3;
+    auto stage = [&](uint32_t r0, uint32_t buf) {
+        for (uint32_t e = threadIdx.x; e < kChunk * kTile / 2u; e += 64u) {
+            const uint32_t r = e / (kTile / 2u), c = e % (kTile / 2u) * 2u;
+            if (r0 + r >= t) break;  // e ascends with r
+            const double *row = xa + (size_t)(r0 + r) * pitch;
+            copy_async16(&si[buf][r][c], row + min(i0 + c, pitch - 2u));
+            copy_async16(&sj[buf][r][c], row + min(j0 + c, pitch - 2u));
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double acc[4][4] = {};
+    stage(0u, 0u);
+    for (uint32_t r0 = 0, buf = 0; r0 < t; r0 += kChunk, buf ^= 1u) {
+        stage(r0 + kChunk, buf ^ 1u);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const uint32_t rn = min(kChunk, t - r0);
+#pragma unroll 4
+        for (uint32_t r = 0; r < rn; ++r) {
+            double iv[4], jv[4];
+            load_spread4<kTile>(si[buf][r], ty, iv);
+            load_spread4<kTile>(sj[buf][r], tx, jv);
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[p][q] = __dadd_rn(acc[p][q], __dmul_rn(iv[p], jv[q]));
+        }
+        __syncthreads();
     }
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t i = i0 + spread4<kTile>(ty, p), j = j0 + spread4<kTile>(tx, q);
+            if (i > f || i > j) continue;
+            if (j < nf) a[(size_t)i * nf + j] = acc[p][q];
+            else if (j == nf) rhs[i] = acc[p][q];
+        }
 }
 
 // a[i][i] += add for every i; with `unbias`, a[f][f] then loses lambda again.
@@ -273,15 +452,78 @@ struct DevBuf {
     }
 };
 
-// G = L L^T in place (lower triangle; n launches of two kernels); true when
-// G is positive definite.
-ne2b_status cholesky(double *g, uint32_t n, unsigned int *bad, cudaStream_t st, bool *pd) {
+// Pinned host memory for a fit's factor, so that its copy runs at the link's
+// rate and the host neither zeroes nor faults in fresh pages.  One buffer of
+// at most kPinnedKeep stays for the next fit of the process; a fit that finds
+// it taken (another thread's) or needs more allocates its own and frees it.
+class PinnedScratch {
+  public:
+    ~PinnedScratch() {
+        if (!p_) return;
+        {
+            std::lock_guard<std::mutex> lk(mu());
+            if (cap_ <= kPinnedKeep && cap_ >= kept().cap) {
+                std::swap(p_, kept().p);
+                std::swap(cap_, kept().cap);
+            }
+        }
+        if (p_) cudaFreeHost(p_);
+    }
+    ne2b_status get(size_t bytes, double **out) {
+        {
+            std::lock_guard<std::mutex> lk(mu());
+            if (kept().cap >= bytes) {
+                std::swap(p_, kept().p);
+                std::swap(cap_, kept().cap);
+            }
+        }
+        if (!p_) {
+            NE2B_CUDA(cudaHostAlloc(&p_, bytes, cudaHostAllocPortable));
+            cap_ = bytes;
+        }
+        *out = (double *)p_;
+        return NE2B_OK;
+    }
+
+  private:
+    static constexpr size_t kPinnedKeep = (size_t)64 << 20;
+    struct Kept {
+        void *p = nullptr;
+        size_t cap = 0;
+    };
+    static std::mutex &mu() {
+        static std::mutex m;
+        return m;
+    }
+    static Kept &kept() {
+        static Kept k;
+        return k;
+    }
+    void *p_ = nullptr;
+    size_t cap_ = 0;
+};
+
+// The default pool keeps up to this much freed memory for the next call
+// (unless it already keeps more): without it each fit maps its workspaces
+// anew.
+void keep_workspace(int device) {
+    cudaMemPool_t pool;
+    uint64_t cur = 0, want = (uint64_t)256 << 20;
+    if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &cur) == cudaSuccess && cur < want)
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &want);
+    cudaGetLastError();
+}
+
+// G = U^T U in place of the upper triangle; true when G is positive definite.
+// dblk: scratch, 32 x 32.
+ne2b_status cholesky(double *g, uint32_t n, double *dblk, unsigned int *bad, cudaStream_t st, bool *pd) {
     NE2B_CUDA(cudaMemsetAsync(bad, 0, sizeof(unsigned int), st));
-    for (uint32_t j = 0; j < n; ++j) {
-        const uint32_t below = n - j - 1u;
-        chol_column_kernel<<<(below + 255) / 256 + (below == 0), 256, 0, st>>>(g, n, j, bad);
-        const dim3 blk(16, 16), grd((below + 15) / 16 + (below == 0), (below + 15) / 16 + (below == 0));
-        chol_update_kernel<<<grd, blk, 0, st>>>(g, n, j, bad);
+    for (uint32_t p = 0; p < n; p += kPanel) {
+        const uint32_t right = n - std::min(n, p + kPanel);  // columns right of the panel
+        chol_panel_kernel<<<std::max(1u, (right + kPanelCols - 1u) / kPanelCols), 32 + kPanelCols, 0, st>>>(g, n, p, dblk, bad);
+        const uint32_t nt = (right + kUpdTile - 1u) / kUpdTile;
+        if (nt) chol_update_kernel<<<nt * (nt + 1u) / 2u, 256, 0, st>>>(g, n, p, dblk, bad);
     }
     NE2B_CUDA(cudaGetLastError());
     unsigned int bad_h = 0;
@@ -289,21 +531,6 @@ ne2b_status cholesky(double *g, uint32_t n, unsigned int *bad, cudaStream_t st, 
     NE2B_CUDA(cudaStreamSynchronize(st));
     *pd = bad_h == 0;
     return NE2B_OK;
-}
-
-// L z = b, L^T w = z with L the lower triangle of l (readout.rs:170-186 order).
-void host_solve(const std::vector<double> &l, const double *b, uint32_t n, double *w) {
-    std::vector<double> z(n);
-    for (uint32_t i = 0; i < n; ++i) {
-        double s = b[i];
-        for (uint32_t q = 0; q < i; ++q) s -= l[(size_t)i * n + q] * z[q];
-        z[i] = s / l[(size_t)i * n + i];
-    }
-    for (uint32_t i = n; i-- > 0;) {
-        double s = z[i];
-        for (uint32_t q = i + 1; q < n; ++q) s -= l[(size_t)q * n + i] * w[q];
-        w[i] = s / l[(size_t)i * n + i];
-    }
 }
 
 // fit_ridge on a device design x[T x F] and host targets y[T].
@@ -319,29 +546,39 @@ ne2b_status fit_binary_on_device(const float *x, uint32_t t, uint32_t f, const f
     NE2B_TRY(buf.get(&b, nf));
     NE2B_TRY(buf.get(&y, t));
     NE2B_TRY(buf.get(&bad, 1));
+    double *dblk = nullptr;
+    NE2B_TRY(buf.get(&dblk, (size_t)kPanel * kPanel));
     NE2B_CUDA(cudaMemcpyAsync(y, y_host, sizeof(float) * t, cudaMemcpyHostToDevice, st));
-    const uint32_t nt = (f + kGramTile - 1) / kGramTile;
-    normal_kernel<<<nt * (nt + 1) / 2, 256, 0, st>>>(x, t, f, a);
-    bias_rhs_kernel<<<(nf + 255) / 256, 256, 0, st>>>(x, y, t, f, a, b);
+    const uint32_t nt = (nf + 1u + kTile - 1u) / kTile;  // columns x, 1 and y
+    const uint32_t pitch = (nf + 2u) / 2u * 2u;
+    double *xa = nullptr;
+    NE2B_TRY(buf.get(&xa, (size_t)t * pitch));
+    for (uint32_t r0 = 0; r0 < t; r0 += 65535u)  // rows along grid y
+        augment_kernel<<<dim3(std::min(64u, (pitch + 255u) / 256u), std::min(65535u, t - r0)), 256, 0, st>>>(
+            x + (size_t)r0 * f, y + r0, t - r0, f, pitch, xa + (size_t)r0 * pitch);
+    normal_kernel<<<nt * (nt + 1) / 2, 64, 0, st>>>(xa, t, f, pitch, a, b);
     const double lam = (double)lambda;
     diag_kernel<<<(nf + 255) / 256, 256, 0, st>>>(a, nf, lam, true, lam);
     NE2B_CUDA(cudaMemcpyAsync(a0, a, sizeof(double) * nf * nf, cudaMemcpyDeviceToDevice, st));
     bool pd = false;
-    NE2B_TRY(cholesky(a, nf, bad, st, &pd));
+    NE2B_TRY(cholesky(a, nf, dblk, bad, st, &pd));
     if (!pd) {  // readout.rs:131-139: more regularisation, once
         NE2B_CUDA(cudaMemcpyAsync(a, a0, sizeof(double) * nf * nf, cudaMemcpyDeviceToDevice, st));
         diag_kernel<<<(nf + 255) / 256, 256, 0, st>>>(a, nf, 1e-3 + lam, false, 0.0);
-        NE2B_TRY(cholesky(a, nf, bad, st, &pd));
+        NE2B_TRY(cholesky(a, nf, dblk, bad, st, &pd));
     }
     if (!pd) {
         for (uint32_t i = 0; i < nf; ++i) w_out[i] = 0.0;
         return NE2B_OK;
     }
-    std::vector<double> l((size_t)nf * nf), bh(nf);
-    NE2B_CUDA(cudaMemcpyAsync(l.data(), a, sizeof(double) * l.size(), cudaMemcpyDeviceToHost, st));
-    NE2B_CUDA(cudaMemcpyAsync(bh.data(), b, sizeof(double) * nf, cudaMemcpyDeviceToHost, st));
+    PinnedScratch pin;
+    double *u = nullptr;
+    NE2B_TRY(pin.get(sizeof(double) * ((size_t)nf * nf + nf), &u));
+    double *bh = u + (size_t)nf * nf;
+    NE2B_CUDA(cudaMemcpyAsync(u, a, sizeof(double) * nf * nf, cudaMemcpyDeviceToHost, st));
+    NE2B_CUDA(cudaMemcpyAsync(bh, b, sizeof(double) * nf, cudaMemcpyDeviceToHost, st));
     NE2B_CUDA(cudaStreamSynchronize(st));
-    host_solve(l, bh.data(), nf, w_out);
+    host_solve1(u, bh, nf, w_out);
     return NE2B_OK;
 }
 
@@ -366,27 +603,40 @@ ne2b_status fit_on_device(const float *x, uint32_t t, uint32_t f, const uint32_t
     NE2B_TRY(buf.get(&a, (size_t)t * k));
     NE2B_TRY(buf.get(&w, (size_t)f * k));
     NE2B_TRY(buf.get(&bad, 1));
-    col_mean_kernel<<<(f + 255) / 256, 256, 0, st>>>(x, t, f, mu);
+    double *dblk = nullptr;
+    NE2B_TRY(buf.get(&dblk, (size_t)kPanel * kPanel));
+    col_mean_kernel<<<(f + 31) / 32, 128, 0, st>>>(x, t, f, mu);
     const uint64_t n = (uint64_t)t * f;
     center_kernel<<<(unsigned)std::min<uint64_t>((n + 255) / 256, 148ull * 64), 256, 0, st>>>(x, n, f, mu, xc);
-    const uint32_t nt = (t + kGramTile - 1) / kGramTile;
-    gram_kernel<<<nt * (nt + 1) / 2, 256, 0, st>>>(xc, t, f, lambda, g);
+    const uint32_t nt = (t + kTile - 1) / kTile;
+    gram_kernel<<<nt * (nt + 1) / 2, 64, 0, st>>>(xc, t, f, lambda, g);
     bool pd = false;
-    NE2B_TRY(cholesky(g, t, bad, st, &pd));
-    // the triangular solves on the host, in the reference's order
-    std::vector<double> L((size_t)t * t), mu_h(f);
-    NE2B_CUDA(cudaMemcpyAsync(L.data(), g, sizeof(double) * L.size(), cudaMemcpyDeviceToHost, st));
+    NE2B_TRY(cholesky(g, t, dblk, bad, st, &pd));
+    // the triangular solves on the host, in the reference's order, four
+    // classes side by side
+    std::vector<double> mu_h(f), ybar(k, 0.0), ah((size_t)t * k, 0.0);
     NE2B_CUDA(cudaMemcpyAsync(mu_h.data(), mu, sizeof(double) * f, cudaMemcpyDeviceToHost, st));
-    NE2B_CUDA(cudaStreamSynchronize(st));
-    std::vector<double> ybar(k, 0.0), ah((size_t)t * k, 0.0), yc(t);
     for (uint32_t r = 0; r < t; ++r) ybar[labels[r]] += 1.0 / (double)t;
-    if (pd)
-        for (uint32_t c = 0; c < k; ++c) {
-            for (uint32_t i = 0; i < t; ++i) yc[i] = (labels[i] == c ? 1.0 : 0.0) - ybar[c];
-            host_solve(L, yc.data(), t, ah.data() + (size_t)c * t);
+    if (pd) {
+        PinnedScratch pin;
+        double *u = nullptr;
+        NE2B_TRY(pin.get(sizeof(double) * (size_t)t * t, &u));
+        NE2B_CUDA(cudaMemcpyAsync(u, g, sizeof(double) * (size_t)t * t, cudaMemcpyDeviceToHost, st));
+        NE2B_CUDA(cudaStreamSynchronize(st));
+        constexpr uint32_t kSide = 4;
+        std::vector<double> yc((size_t)t * kSide), ac((size_t)t * kSide);
+        for (uint32_t c0 = 0; c0 < k; c0 += kSide) {
+            for (uint32_t i = 0; i < t; ++i)
+                for (uint32_t c = 0; c < kSide; ++c)
+                    yc[(size_t)i * kSide + c] =
+                        c0 + c < k ? (labels[i] == c0 + c ? 1.0 : 0.0) - ybar[c0 + c] : 0.0;
+            host_solve4(u, yc.data(), t, ac.data());
+            for (uint32_t c = 0; c < kSide && c0 + c < k; ++c)
+                for (uint32_t i = 0; i < t; ++i) ah[(size_t)(c0 + c) * t + i] = ac[(size_t)i * kSide + c];
         }
+    }
     NE2B_CUDA(cudaMemcpyAsync(a, ah.data(), sizeof(double) * ah.size(), cudaMemcpyHostToDevice, st));
-    weights_kernel<<<dim3((f + 255) / 256, k), 256, 0, st>>>(xc, a, t, f, k, w);
+    weights_kernel<<<dim3((f + 31) / 32, (k + 3) / 4), 32, 0, st>>>(xc, a, t, f, k, w);
     NE2B_CUDA(cudaGetLastError());
     std::vector<double> wh((size_t)f * k);
     NE2B_CUDA(cudaMemcpyAsync(wh.data(), w, sizeof(double) * wh.size(), cudaMemcpyDeviceToHost, st));
@@ -423,6 +673,7 @@ ne2b_status ne2b_fit_ridge_multi(const float *x, uint32_t t, uint32_t f, const u
         cudaStream_t st = nullptr;
         e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
         if (e != cudaSuccess) return ne2b::cuda_error(e, "cudaStreamCreate");
+        ne2b::keep_workspace(device);
         ne2b_status r = NE2B_OK;
         {
             ne2b::DevBuf buf(st);
@@ -517,6 +768,7 @@ ne2b_status ne2b_fit_ridge(const float *x, uint32_t t, uint32_t f, const float *
         cudaStream_t st = nullptr;
         e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
         if (e != cudaSuccess) return ne2b::cuda_error(e, "cudaStreamCreate");
+        ne2b::keep_workspace(device);
         ne2b_status r = NE2B_OK;
         {
             ne2b::DevBuf buf(st);

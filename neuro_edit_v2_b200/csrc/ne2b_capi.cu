@@ -143,6 +143,7 @@ static ne2b_status create_from_list(ne2b::Engine &eng, const ne2b_net_desc *net,
     if (d_dly) dc.syn.delay_ms = dly; else { LIST_TRY(dalloc(4 * E, &p)); dc.syn.delay_ms = (const float *)p; }
     if (d_kind) dc.syn.kind = kind; else { LIST_TRY(dalloc(n, &p)); dc.syn.kind = (const uint8_t *)p; }
     LIST_TRY(dalloc(2 * E, &p)); dc.steps = (const uint16_t *)p;
+    LIST_TRY(dalloc(4 * E, &p)); dc.place = (const uint32_t *)p;
     LIST_TRY(dalloc(4 * (size_t)n, &p)); dc.counts = (const uint32_t *)p;
     LIST_TRY(dalloc(4 * (size_t)n, &p)); dc.cursor = (uint32_t *)p;
     LIST_TRY(dalloc(4 * (size_t)csr_scan_blocks(n), &p)); dc.sums = (uint32_t *)p;
@@ -153,7 +154,7 @@ static ne2b_status create_from_list(ne2b::Engine &eng, const ne2b_net_desc *net,
     dc.syn.n_syn = E;
     dc.syn.n = n;
     dc.syn.dt_ms = cfg->dt_ms;
-    CsrScalars sc{~0ull, ~0ull, 1u, ~0u, 0u};
+    CsrScalars sc{~0ull, ~0ull, 1u, ~0u, 0u, 0u};
     if (E) {
         if (!d_src) LIST_TRY(eng.pin_copy((void *)dc.syn.src, src, 4 * E));
         if (!d_tgt) LIST_TRY(eng.pin_copy((void *)dc.syn.tgt, tgt, 4 * E));
@@ -165,7 +166,7 @@ static ne2b_status create_from_list(ne2b::Engine &eng, const ne2b_net_desc *net,
     LIST_TRY(eng.pin_close());
     LIST_TRY(cuda_error(cudaMemsetAsync((void *)dc.counts, 0, 4 * (size_t)n, st), "memset counts"));
     LIST_TRY(cuda_error(cudaMemsetAsync(dc.ticket, 0, 4 * (chunks + 1), st), "memset tickets"));
-    LIST_TRY(cuda_error(csr_prepass(dc.syn, (uint32_t *)dc.counts, (uint16_t *)dc.steps, dc.sc, st), "csr prepass"));
+    LIST_TRY(cuda_error(csr_prepass(dc.syn, (uint32_t *)dc.counts, (uint32_t *)dc.place, (uint16_t *)dc.steps, dc.sc, st), "csr prepass"));
     LIST_TRY(cuda_error(cudaMemcpyAsync(&sc, dc.sc, sizeof sc, cudaMemcpyDeviceToHost, st), "prepass readback"));
     LIST_TRY(cuda_error(cudaStreamSynchronize(st), "prepass"));
     if (sc.bad_ref != ~0ull) {
@@ -183,6 +184,7 @@ static ne2b_status create_from_list(ne2b::Engine &eng, const ne2b_net_desc *net,
     }
     dc.max_delay = sc.max_delay;
     dc.min_delay = sc.min_delay;
+    dc.short_rows = csr_rows_short(sc.max_row);
     LIST_TRY(eng.add_net_device_csr(net, cfg, dc, slot));
     LIST_TRY(cuda_error(cudaMemcpyAsync(&sc, dc.sc, sizeof sc, cudaMemcpyDeviceToHost, st), "scatter readback"));
     LIST_TRY(cuda_error(cudaStreamSynchronize(st), "device CSR build"));

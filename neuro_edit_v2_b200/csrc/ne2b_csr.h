@@ -25,12 +25,22 @@ struct CsrScalars {
     unsigned long long bad_delay;  // first synapse whose delay exceeds 65535 steps
     uint32_t max_delay;            // largest delay in steps (>= 1)
     uint32_t min_delay;            // smallest delay in steps (~0 without synapses)
+    uint32_t max_row;              // synapses of the source with the most
     uint32_t timeout;              // a scatter block gave up waiting for its predecessor
 };
 
 // Checks references, rounds delays to steps, counts synapses per source
-// (counts zeroed by the caller) and finds the largest delay.
-cudaError_t csr_prepass(const DevSynapses &ds, uint32_t *counts, uint16_t *steps, CsrScalars *sc, cudaStream_t st);
+// (counts zeroed by the caller), gives each synapse a place of its own in its
+// source's row (place[n_syn], in no particular order) and finds the largest
+// and smallest delay and the longest row.
+cudaError_t csr_prepass(const DevSynapses &ds, uint32_t *counts, uint32_t *place, uint16_t *steps, CsrScalars *sc,
+                        cudaStream_t st);
+// Rows short enough for csr_place_and_order (16 bytes of scratch per
+// synapse); else csr_scatter.
+bool csr_rows_short(uint32_t max_row);
+cudaError_t csr_place_and_order(const DevSynapses &ds, const uint16_t *steps, const uint32_t *place,
+                                const uint32_t *rowptr, void *scratch, SynRec *syn_out, uint16_t *delay16_out,
+                                bool int_w, bool wide, cudaStream_t st);
 // Row pointers [n + 1] from the counts; cursor [n] = rowptr[0..n).  `sums`
 // holds csr_scan_blocks(n) words.
 cudaError_t csr_scan(const uint32_t *counts, uint32_t n, uint32_t e, uint32_t *rowptr, uint32_t *cursor,

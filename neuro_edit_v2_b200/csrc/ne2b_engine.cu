@@ -120,13 +120,15 @@ ne2b_status Engine::init(int device, bool int_ring, uint32_t max_nets) {
     device_ = device;
     int_ring_ = int_ring;
     NE2B_CUDA(cudaSetDevice(device));
-    cudaDeviceProp prop;
-    NE2B_CUDA(cudaGetDeviceProperties(&prop, device));
-    if (prop.major < 10)
-        return set_error(NE2B_UNSUPPORTED, "device %d is sm_%d%d; this library is built for sm_100a", device,
-                         prop.major, prop.minor);
+    // single attributes: the whole property record takes 2.6 ms to read
+    int major = 0, minor = 0;
+    NE2B_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+    NE2B_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+    if (major < 10)
+        return set_error(NE2B_UNSUPPORTED, "device %d is sm_%d%d; this library is built for sm_100a", device, major,
+                         minor);
     noalloc_setup(device);  // scratch address of ne2b_spike_counts_noalloc; a failure only disables that entry point
-    sm_count_ = prop.multiProcessorCount;
+    NE2B_CUDA(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device));
     NE2B_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     stager_.set_stream(stream_);
     {
@@ -319,7 +321,8 @@ ne2b_status Stager::reserve(size_t bytes, void **host) {
         }
         if (cur_ < 0) {
             PinnedBlock b;
-            b.cap = std::max<size_t>(need, (size_t)64 << 20);
+            // what this net needs, at least 4 MB: pinning costs 0.25 ms per MB
+            b.cap = std::max<size_t>(need, (size_t)4 << 20);
             NE2B_CUDA(cudaMallocHost(&b.p, b.cap));
             NE2B_CUDA(cudaEventCreateWithFlags(&b.ev, cudaEventDisableTiming));
             pin_.push_back(b);
@@ -570,10 +573,20 @@ ne2b_status Engine::build_net(const ne2b_net_desc *net, const ne2b_config *cfg, 
         // the list's CSR sorted into place on the device (csrc/ne2b_csr.cu)
         NET_TRY(cuda_error(csr_scan(dc->counts, n, (uint32_t)h->e, (uint32_t *)d.rowptr, dc->cursor, dc->sums, bst),
                            "device CSR: row pointers"));
+        if (dc->short_rows) {
+            void *scratch = nullptr;
+            if (h->e) {
+                NET_TRY(cuda_error(cudaMallocAsync(&scratch, 16 * (size_t)h->e, bst), "cudaMallocAsync (device CSR)"));
+                const cudaError_t e = csr_place_and_order(dc->syn, dc->steps, dc->place, d.rowptr, scratch, (SynRec *)d.syn,
+                                                          (uint16_t *)d.delay16, int_ring_, wide, bst);
+                cudaFreeAsync(scratch, bst);
+                NET_TRY(cuda_error(e, "device CSR: place and order"));
+            }
+        } else
         NET_TRY(cuda_error(csr_scatter(dc->syn, dc->steps, dc->cursor, (SynRec *)d.syn, (uint16_t *)d.delay16, int_ring_, wide,
                                        dc->ticket, dc->done, dc->sc, 5000000000ull, bst),
                            "device CSR: scatter"));
-        h->build_launches += (n ? 3 : 0) + (h->e ? 1 : 0);
+        h->build_launches += (n ? 3 : 0) + (h->e ? (dc->short_rows ? 2 : 1) : 0);
     } else {
         NET_TRY(up((void *)d.rowptr, net->src_ptr, sizeof(uint32_t) * ((size_t)n + 1)));
     }

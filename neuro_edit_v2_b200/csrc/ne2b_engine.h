@@ -29,6 +29,8 @@ struct DevCsrBuild {
     const uint16_t *steps = nullptr;   // delay steps per list entry
     const uint32_t *counts = nullptr;  // synapses per source
     uint32_t max_delay = 1, min_delay = ~0u;
+    const uint32_t *place = nullptr;   // each synapse's place in its row
+    bool short_rows = true;            // csr_rows_short: place and order; else scatter
     uint32_t *cursor = nullptr;        // [n]
     uint32_t *sums = nullptr;          // [csr_scan_blocks(n)]
     uint32_t *ticket = nullptr;        // [1], zeroed

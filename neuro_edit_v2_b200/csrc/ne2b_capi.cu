@@ -479,7 +479,7 @@ ne2b_status ne2b_set_delivery_warps(ne2b_sim *sim, int32_t on) {
 ne2b_status ne2b_delivery_warps(ne2b_sim *sim, int32_t *on, int32_t *active) {
     if (!sim || !on || !active) return set_error(NE2B_EINVAL, "null argument");
     *on = sim->eng.shape().ws ? 1 : 0;
-    *active = (!sim->eng.resident() && !sim->eng.cluster() && sim->eng.ws_applies(sim->eng.shape())) ? 1 : 0;
+    *active = (!sim->eng.resident() && !sim->eng.cluster() && !sim->eng.deferred() && sim->eng.ws_applies(sim->eng.shape())) ? 1 : 0;
     return NE2B_OK;
 }
 

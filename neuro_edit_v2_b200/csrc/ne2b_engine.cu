@@ -1014,6 +1014,8 @@ ne2b_status Engine::choose_kernel() {
     if (!plan_stale_) return NE2B_OK;
     std::vector<ClusterNet> plan;
     cluster_ = !resident_ && plan_cluster(plan);
+    if (!cluster_ && !resident_) NE2B_TRY(plan_defer());
+    if (defer_) NE2B_TRY(build_tiles(defer_shape_));
     if (cluster_) {
         if (!d_plan_) NE2B_CUDA(cudaMalloc(&d_plan_, sizeof(ClusterNet) * nets_cap_));
         // pageable source, staged by the runtime before the call returns
@@ -1053,8 +1055,70 @@ ne2b_status Engine::launch_clusters(uint32_t steps) {
     return NE2B_OK;
 }
 
+// Delivery blocks of the deferred-delivery kernel for a net of n neurons:
+// one per 512 neurons, up to one per SM (100k neurons at 25 Hz list 250
+// spikes per step; 74, 148 and 296 blocks: 3.28, 3.27 and 3.31 us).
+static uint32_t deliver_blocks(uint32_t n, int sm_count) {
+    return std::max(1u, std::max((uint32_t)sm_count / 4u, std::min((uint32_t)sm_count, n / 512u)));
+}
+
+// Deferred delivery (step_kernel_defer): one net on the streaming kernel with
+// no tile shape asked for, whose tiles of 128 neurons run in one wave beside
+// the delivery blocks (132k neurons on 148 SMs).  Measured per step, 128 x 1
+// tiles, deferred against the fused kernel's best shape: 100k quiet 1.78 /
+// 1.82 us, active 3.2 / 3.9; AdEx 2.20 / 2.23, 4.5 / 4.8; 20k 1.48 / 1.66, 2.6
+// / 3.2.  Past one wave it loses its point: the neuron pass takes longer than
+// the delivery it hides, and the fused kernel's larger tiles win (200k 2.8 /
+// 2.4, 5.8 / 5.3; 1M 8.9 / 6.4).  Not taken when more than one neuron in 16
+// has a synapse of delay 1: their rows would be read twice, a warp at a time.
+ne2b_status Engine::plan_defer() {
+    if (mode_ != kModeAuto || shape_set_ || multi_net || active_nets() != 1) return NE2B_OK;
+    NetHost *h = nullptr;
+    for (NetHost *x : nets_)
+        if (x) h = x;
+    if (!h->n) return NE2B_OK;
+    defer_shape_.block = kDeferBlock;
+    defer_shape_.npt = 1;
+    const uint32_t occ = (uint32_t)defer_occupancy(int_ring_, adex_, false);
+    if (h->n_pad / kDeferBlock + 1u + deliver_blocks(h->n, sm_count_) > occ * (uint32_t)sm_count_) return NE2B_OK;
+    NetDev &d = h->dev;
+    if (h->urgent < 0) {  // once per net
+        void *p = nullptr;
+        h->urgent = 0;
+        if (d.hop == 1u) {
+            const size_t words = h->n_pad / 32 + 1;  // the last one counts
+            NE2B_CUDA(cudaMallocAsync(&p, sizeof(uint32_t) * words, stream_));
+            h->allocs.push_back(p);
+            uint32_t *bits = (uint32_t *)p, count = 0;
+            NE2B_CUDA(cudaMemsetAsync(bits, 0, sizeof(uint32_t) * words, stream_));
+            NE2B_CUDA(launch_urgent(d, bits, bits + words - 1, stream_));
+            launches_ += 1;
+            NE2B_CUDA(cudaMemcpyAsync(&count, bits + words - 1, sizeof count, cudaMemcpyDeviceToHost, stream_));
+            NE2B_CUDA(cudaStreamSynchronize(stream_));
+            h->urgent = (int64_t)count;
+            d.urgent = bits;
+        }
+        if (h->urgent * 16 <= (int64_t)h->n) {
+            NE2B_CUDA(cudaMallocAsync(&p, sizeof(uint2_pod) * 3 * (size_t)h->n_pad + 16, stream_));
+            h->allocs.push_back(p);
+            d.slist = (uint2_pod *)p;
+            d.scount = (uint32_t *)(d.slist + 3 * (size_t)h->n_pad);
+        }
+        NE2B_TRY(upload_net(*h));
+    }
+    if (!d.slist) return NE2B_OK;
+    defer_ = true;
+    return NE2B_OK;
+}
+
 ne2b_status Engine::rebuild_tiles() {
-    const uint32_t tile = shape_.block * shape_.npt;
+    plan_stale_ = true;
+    defer_ = false;  // chosen again, with its own tiles, when steps are next run
+    return build_tiles(shape_);
+}
+
+ne2b_status Engine::build_tiles(const TileShape &shape) {
+    const uint32_t tile = shape.block * shape.npt;
     std::vector<Tile> tiles;
     bool adex = false;
     for (NetHost *h : nets_)
@@ -1084,7 +1148,6 @@ ne2b_status Engine::rebuild_tiles() {
     const uint32_t old_grid = grid();
     std::vector<uint32_t> block_tiles;
     resident_ = plan_resident(tiles, block_tiles);
-    plan_stale_ = true;
     if (mode_ == kModeResident && !resident_ && !tiles.empty())
         return set_error(NE2B_UNSUPPORTED, "the nets do not fit the resident kernel's shared memory");
     if (tiles.size() > tiles_cap_ || block_tiles.size() > block_tiles_cap_) NE2B_CUDA(cudaStreamSynchronize(stream_));
@@ -1270,6 +1333,7 @@ ne2b_status Engine::launch_group(uint32_t steps) {
         return NE2B_OK;
     }
     if (cluster_) return launch_clusters(steps);
+    if (defer_) return launch_deferred(steps);
     // the instance follows the nets' features (an external current or a
     // watch can be switched on and off between launches)
     const int var = step_variant();
@@ -1303,6 +1367,50 @@ ne2b_status Engine::launch_group(uint32_t steps) {
     for (uint32_t k = 0; k < steps; ++k) NE2B_CUDA(launch_step(int_ring_, adex_, var, shape_.block, shape_.npt, d_eng_, k, g, stream_));
     NE2B_CUDA(launch_advance(d_nets_, nets_cap_, steps, stream_));
     launches_ += steps + 1;
+    return NE2B_OK;
+}
+
+// A launch group on the deferred-delivery kernel: the counts cleared, the
+// steps, the last list's flush, the advance; from a graph at graph_steps.
+ne2b_status Engine::launch_deferred(uint32_t steps) {
+    NetHost *h = nullptr;
+    for (NetHost *x : nets_)
+        if (x) h = x;
+    const bool plain = step_variant(TileShape{}) == kStepPlain;
+    const int var = 0x100 | (plain ? 1 : 0);
+    if (var != graph_variant_) {
+        clear_graphs();
+        graph_variant_ = var;
+    }
+    const uint32_t nd = deliver_blocks(h->n, sm_count_), grid = nd + n_tiles_;  // one tile per block (plan_defer)
+    auto group = [&]() -> cudaError_t {
+        cudaError_t e = cudaMemsetAsync(h->dev.scount, 0, 3 * sizeof(uint32_t), stream_);
+        for (uint32_t k = 0; k < steps && e == cudaSuccess; ++k)
+            e = launch_defer(int_ring_, adex_, plain, d_eng_, nd, k, grid, stream_);
+        if (e == cudaSuccess) e = launch_defer_flush(int_ring_, adex_, d_eng_, nd, steps, stream_);
+        if (e == cudaSuccess) e = launch_advance(d_nets_, nets_cap_, steps, stream_);
+        return e;
+    };
+    launches_ += steps + 2;
+    if (steps != graph_steps) {
+        NE2B_CUDA(group());
+        return NE2B_OK;
+    }
+    auto it = graphs_.find(steps);
+    if (it == graphs_.end()) {
+        cudaGraph_t gr;
+        NE2B_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+        const cudaError_t err = group();
+        const cudaError_t e2 = cudaStreamEndCapture(stream_, &gr);
+        if (err != cudaSuccess) return cuda_error(err, "step launch during capture");
+        NE2B_CUDA(e2);
+        cudaGraphExec_t ex;
+        const cudaError_t e3 = cudaGraphInstantiate(&ex, gr, 0);
+        cudaGraphDestroy(gr);
+        NE2B_CUDA(e3);
+        it = graphs_.emplace(steps, ex).first;
+    }
+    NE2B_CUDA(cudaGraphLaunch(it->second, stream_));
     return NE2B_OK;
 }
 
@@ -1650,6 +1758,12 @@ void Engine::drop(EngineSnapshot &snap) {
 // occupancy, the resident kernel wherever its shared-memory plan fits.
 ne2b_status Engine::autotune(uint32_t steps_per_trial) {
     if (steps_per_trial == 0) steps_per_trial = graph_steps;
+    // what the automatic choice allocates has to be there before the snapshot
+    if (mode_ == kModeAuto) {
+        shape_set_ = false;
+        NE2B_TRY(rebuild_tiles());
+        NE2B_TRY(choose_kernel());
+    }
     EngineSnapshot snap;
     NE2B_TRY(snapshot(snap));
     // bring the clocks up from idle and size the trials: every candidate runs
@@ -1671,7 +1785,7 @@ ne2b_status Engine::autotune(uint32_t steps_per_trial) {
     uint32_t blocks[32], npts[32], count = 0;
     shape_list(blocks, npts, &count);
     const int saved_mode = mode_;
-    bool best_cluster = false;
+    bool best_auto = false;
     TileShape best = shape_;
     int best_mode = mode_ == kModeAuto ? (resident_ ? kModeResident : kModeStream) : mode_;
     float best_ms = 1e30f;
@@ -1692,13 +1806,13 @@ ne2b_status Engine::autotune(uint32_t steps_per_trial) {
         }
         return NE2B_OK;
     };
-    if (saved_mode == kModeAuto) {  // the cluster kernel, where it applies
+    if (saved_mode == kModeAuto) {  // the cluster or deferred-delivery kernel, where one applies
         shape_set_ = false;
         NE2B_TRY(rebuild_tiles());
         NE2B_TRY(choose_kernel());
-        if (cluster_) {
+        if (cluster_ || defer_) {
             NE2B_TRY(trial(&best_ms));
-            best_cluster = true;
+            best_auto = true;
         }
     }
     shape_set_ = true;
@@ -1723,16 +1837,16 @@ ne2b_status Engine::autotune(uint32_t steps_per_trial) {
                 NE2B_TRY(trial(&ms));
                 if (ms < best_ms) {
                     best_ms = ms;
-                    best_cluster = false;
+                    best_auto = false;
                     best = s;
                     best_mode = m;
                 }
             }
         }
     }
-    mode_ = saved_mode == kModeAuto && !best_cluster ? best_mode : saved_mode;
+    mode_ = saved_mode == kModeAuto && !best_auto ? best_mode : saved_mode;
     shape_ = best;
-    shape_set_ = !best_cluster;
+    shape_set_ = !best_auto;
     clear_graphs();
     NE2B_TRY(rebuild_tiles());
     NE2B_TRY(restore(snap));

@@ -58,6 +58,7 @@ struct NetHost {
     uint32_t slot = 0;        // index in the engine's net array
     uint32_t n = 0, n_pad = 0, D = 0, n_inputs = 0;
     uint64_t e = 0;
+    int64_t urgent = -1;      // neurons with a synapse of delay 1, -1 before they are counted
     uint32_t nx = 0;          // synapses with their own tau (XSyn)
     uint64_t t = 0;           // host mirror of dev.t
     uint64_t t_end = ~0ull;
@@ -222,6 +223,7 @@ class Engine {
     bool resident() const { return resident_; }
     // the cluster kernel runs the next steps (ne2b_cluster.cuh)
     bool cluster() { return choose_kernel() == NE2B_OK && cluster_; }
+    bool deferred() { return choose_kernel() == NE2B_OK && defer_; }
     int mode() const { return mode_; }
     ne2b_status set_mode(int m);
     // the streaming kernel runs separate delivery warps for shape `s`
@@ -244,6 +246,9 @@ class Engine {
     int step_variant() const;
     int step_variant(const TileShape &s) const;  // with `s`'s delivery warps where they apply
     ne2b_status choose_kernel();
+    ne2b_status plan_defer();
+    ne2b_status launch_deferred(uint32_t steps);
+    ne2b_status build_tiles(const TileShape &shape);
     struct ClusterClass {  // nets with the same cluster size and kind of hop: one launch
         uint32_t blocks, smem, first, count;
         ClusterShape shape;
@@ -288,6 +293,8 @@ class Engine {
     bool resident_ = false;
     bool adex_ = false;  // some net holds AdEx rows: the kernels with the AdEx path run
     // cluster kernel
+    bool defer_ = false;       // the deferred-delivery kernel runs, on tiles of defer_shape_
+    TileShape defer_shape_;
     bool cluster_ = false;
     bool plan_stale_ = true;  // the nets or the kernel choice changed since the plan was made
     bool shape_set_ = false;  // a tile shape was chosen: the streaming kernel runs with it

@@ -64,6 +64,21 @@ __global__ void pn_total_kernel(const unsigned long long *pn, uint32_t n, uint32
     out[i] = c > 0xffffffffull ? 0xffffffffu : (uint32_t)c;
 }
 
+// A warp per row: does it hold a synapse of delay 1?
+__global__ void urgent_kernel(NetDev nd, uint32_t *bits, uint32_t *count) {
+    const uint32_t lane = threadIdx.x & 31u, nw = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < nd.n; i += nw) {
+        const uint32_t lo = nd.rowptr[i], hi = nd.rowptr[i + 1];
+        bool one = false;
+        for (uint32_t j = lo + lane; j < hi; j += 32u)
+            one |= ((nd.flags & kNetDelayWide) ? (uint32_t)nd.delay16[j] : nd.syn[j].td >> kSynTgtBits) == 1u;
+        if (__any_sync(0xffffffffu, one) && lane == 0u) {
+            atomicOr(bits + (i >> 5), 1u << (i & 31u));
+            atomicAdd(count, 1u);
+        }
+    }
+}
+
 // Self-test of the bounded grid barrier: every block but `absent` arrives,
 // so the others give up after `limit_ns`, set the error flag and return
 // (a wait that cannot end, ended by its limit, with no fault).
@@ -130,6 +145,27 @@ int resident_occupancy(bool int_ring, bool adex, uint32_t block, uint32_t npt, s
 cudaError_t launch_resident(bool int_ring, bool adex, uint32_t block, uint32_t npt, const EngineDev *eng,
                             uint32_t k0, uint32_t nsteps, uint32_t grid, size_t smem, cudaStream_t st) {
     return NE2B_KIND(int_ring, adex, launch_resident(block, npt, eng, k0, nsteps, grid, smem, st));
+}
+
+int defer_occupancy(bool int_ring, bool adex, bool plain) {
+    return NE2B_KIND(int_ring, adex, defer_occupancy(plain));
+}
+
+cudaError_t launch_defer(bool int_ring, bool adex, bool plain, const EngineDev *eng, uint32_t n_deliver,
+                         uint32_t k_step, uint32_t grid, cudaStream_t st) {
+    return NE2B_KIND(int_ring, adex, launch_defer(plain, eng, n_deliver, k_step, grid, st));
+}
+
+cudaError_t launch_defer_flush(bool int_ring, bool adex, const EngineDev *eng, uint32_t n_deliver, uint32_t steps,
+                               cudaStream_t st) {
+    return NE2B_KIND(int_ring, adex, launch_defer_flush(eng, n_deliver, steps, st));
+}
+
+cudaError_t launch_urgent(const NetDev &nd, uint32_t *bits, uint32_t *count, cudaStream_t st) {
+    if (nd.n == 0) return cudaSuccess;
+    const uint32_t blocks = (nd.n + 7u) / 8u;
+    urgent_kernel<<<blocks < 148u * 32u ? blocks : 148u * 32u, 256, 0, st>>>(nd, bits, count);
+    return cudaGetLastError();
 }
 
 int cluster_fit(bool int_ring, bool adex, bool full, uint32_t blocks, const ClusterShape &cs, size_t smem) {

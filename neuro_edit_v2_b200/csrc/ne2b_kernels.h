@@ -27,6 +27,16 @@ uint32_t resident_head(uint32_t block, uint32_t npt);
 int resident_occupancy(bool int_ring, bool adex, uint32_t block, uint32_t npt, size_t smem);
 cudaError_t launch_resident(bool int_ring, bool adex, uint32_t block, uint32_t npt, const EngineDev *eng,
                             uint32_t k0, uint32_t nsteps, uint32_t grid, size_t smem, cudaStream_t st);
+// Deferred-delivery kernel (step_kernel_defer): `grid` blocks, the first
+// `n_deliver` of which deliver; after a group's steps, the flush.
+int defer_occupancy(bool int_ring, bool adex, bool plain);
+cudaError_t launch_defer(bool int_ring, bool adex, bool plain, const EngineDev *eng, uint32_t n_deliver,
+                         uint32_t k_step, uint32_t grid, cudaStream_t st);
+cudaError_t launch_defer_flush(bool int_ring, bool adex, const EngineDev *eng, uint32_t n_deliver, uint32_t steps,
+                               cudaStream_t st);
+// bits[i / 32] bit i % 32: neuron i has a synapse of delay 1; *count += such
+// neurons (both zeroed by the caller).
+cudaError_t launch_urgent(const NetDev &nd, uint32_t *bits, uint32_t *count, cudaStream_t st);
 // Cluster kernel (ne2b_cluster.cuh): co-resident clusters (0: it does not
 // fit), and one launch of `clusters` nets for `steps` steps, t included.
 int cluster_fit(bool int_ring, bool adex, bool full, uint32_t blocks, const ClusterShape &cs, size_t smem);

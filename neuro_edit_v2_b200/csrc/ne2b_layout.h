@@ -77,6 +77,10 @@ constexpr uint32_t kNeverSpiked = 0xFFFFFFFFu;  // gw_ls of a texel that never s
 constexpr uint32_t kParamAdexBit = 0x8000u;  // pidx bit: the row is an AdEx row
 constexpr uint32_t kSmemParamRows = 32;      // param tables up to this size are staged in shared memory
 
+struct alignas(8) uint2_pod {
+    uint32_t x, y;
+};
+
 // Per-network descriptor.  Device copy read by the kernels; the host keeps a
 // mirror and rewrites the fields it changes.
 struct alignas(16) NetDev {
@@ -117,6 +121,12 @@ struct alignas(16) NetDev {
     const int32_t *gw_map;      // [gw_n][n_pad] member-list position of neuron i in group g, or -1
     const uint32_t *gw_off;     // [gw_n + 1] group ranges in gw_ls
     uint32_t *gw_ls;            // last spike step per texel (min(t, 2^32-2)), kNeverSpiked
+    // deferred delivery (step_kernel_defer): three spike lists of {row start,
+    // row end}, one per step in turn, n_pad entries each, and their counts;
+    // urgent: one bit per neuron with a synapse of delay 1, or null
+    uint2_pod *slist;
+    uint32_t *scount;
+    const uint32_t *urgent;
     uint32_t watch_n, gw_n;
     // scalars
     unsigned long long t;       // step index of the next launch group's k = 0

@@ -140,11 +140,51 @@ __device__ __forceinline__ void ring_add(uint32_t *word, uint32_t wb, uint64_t p
                       : "memory");
 }
 
+// A listed row's synapses (those of delay 1 when `first`, else the others
+// when the net has urgent neurons), strided by a warp, four per lane and pass
+// with their loads in flight before the adds, into slot (ts + delay) % D.
+template <bool INT, bool XSYN>
+__device__ __forceinline__ void defer_deliver(const NetDev &nd, uint32_t rlo, uint32_t len, uint32_t ts, uint32_t lane,
+                                              bool first, uint64_t pol) {
+    constexpr int U = 4;
+    const uint32_t D = nd.D, n_pad = nd.n_pad, flags = nd.flags;
+    const bool wide = flags & kNetDelayWide, skip = nd.urgent != nullptr;
+    uint32_t *__restrict__ ringw = (uint32_t *)nd.ring;
+    const SynRec *__restrict__ csr = nd.syn + rlo;
+    for (uint32_t f = lane; f < len; f += 32u * U) {
+        uint2 r[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            r[q] = *reinterpret_cast<const uint2 *>(csr + (f + 32u * q < len ? f + 32u * q : f));
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const uint32_t j = f + 32u * q;
+            if (j >= len) continue;
+            const uint32_t d = wide ? (uint32_t)nd.delay16[rlo + j] : r[q].x >> kSynTgtBits;
+            if (first ? d != 1u : (skip && d == 1u)) continue;
+            uint32_t slot = ts + d;
+            if (slot >= D) slot -= D;
+            if (XSYN && (flags & kNetXsyn)) {
+                const uint32_t xk = nd.xmap[rlo + j];
+                if (xk != kNoXsyn) {  // its own current: mark the arrival (cpu.rs:270-273)
+                    atomicOr(nd.xpend + (size_t)slot * nd.xwords + (xk >> 5), 1u << (xk & 31u));
+                    continue;
+                }
+            }
+            const uint32_t tg = wide ? r[q].x : r[q].x & kSynTgtMask;
+            ring_add<INT>(ringw + (size_t)slot * n_pad + tg, r[q].y, pol);
+        }
+    }
+}
+
 // WSQ (step_kernel_ws): the tile's threads are the producer warps of a
 // delivery queue; they push their spiking neurons' rows into `wq` and count
 // their spikes into *nspk (per warp) instead of compacting and delivering.
+// DEFER (step_kernel_defer): each warp appends its spiking neurons' rows to
+// the step's spike list, which the next step's delivery blocks take, and
+// delivers at once only synapses of delay 1.
 template <bool INT, int BLOCK, int NPT, bool RES, bool ADEX, bool PHASES, bool LEAN = false, bool NOIO = false,
-          bool WSQ = false>
+          bool WSQ = false, bool DEFER = false>
 __device__ __forceinline__ void process_tile(const EngineDev *__restrict__ eng, const ParamRow *ptab, const NetDev &nd,
                                              const Tile &tile, uint64_t t, uint32_t tmod, uint32_t k, float *vs, float *us,
                                              float *ss, uint16_t *tks, const uint16_t *pis, const SmemLists &sl,
@@ -352,6 +392,29 @@ __device__ __forceinline__ void process_tile(const EngineDev *__restrict__ eng, 
             const uint32_t off = q * BLOCK + warp * 32;
             if (lane == 0 && off < tile.count) nd.rec_bits[(size_t)row * words32 + ((tile.start + off) >> 5)] = mask;
         }
+    }
+    if constexpr (DEFER) {
+        const uint32_t lt = (1u << lane) - 1u;
+        const uint32_t which = k % 3u;
+#pragma unroll
+        for (int q = 0; q < NPT; ++q) {
+            const uint32_t m = __ballot_sync(0xffffffffu, spk[q]);
+            if (m == 0u) continue;
+            const int leader = __ffs(m) - 1;
+            uint32_t base = 0;
+            if (lane == leader) base = atomicAdd(nd.scount + which, (uint32_t)__popc(m));
+            const uint32_t urg = nd.urgent ? m & nd.urgent[(tile.start + q * BLOCK + warp * 32) >> 5] : 0u;
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (spk[q])
+                *reinterpret_cast<uint2 *>(nd.slist + (size_t)which * n_pad + base + __popc(m & lt)) =
+                    make_uint2(rlo[q], rhi[q]);
+            for (uint32_t u = urg; u; u &= u - 1u) {  // rare: the row's synapses of delay 1, now
+                const int l = __ffs(u) - 1;
+                const uint32_t lo = __shfl_sync(0xffffffffu, rlo[q], l), hi = __shfl_sync(0xffffffffu, rhi[q], l);
+                defer_deliver<INT, !LEAN>(nd, lo, hi - lo, tmod, lane, true, ring_policy());
+            }
+        }
+        return;
     }
     if constexpr (WSQ) {
         // ---- push each spiking neuron's CSR row to the block's delivery
@@ -667,6 +730,79 @@ template <bool INT, int BLOCK, bool ADEX>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) step_kernel_r64(const EngineDev *__restrict__ eng,
                                                                        uint32_t k_step) {
     step_body<INT, BLOCK, 1, ADEX, false, true>(eng, k_step);
+}
+
+// -------------------------------------- streaming kernel, delivery deferred
+// One net.  The launch of step t holds two kinds of blocks: the first
+// `n_deliver` blocks deliver the spikes of step t - 1 (their list was
+// complete when the launch began), the others do step t's neuron pass and
+// list its spikes.  Delivery so overlaps the next step's neuron pass instead
+// of following its own tile's: the active step's chain (state, neuron pass,
+// row pointers, block scan, CSR, adds) becomes two shorter ones side by side.
+// It may wait a step because only a synapse of delay 1 lands in the next
+// step's slot; a neuron that has one (a bit in nd.urgent, loaded only when
+// its warp spikes) delivers those at once.  The tile blocks need no block
+// barrier at all.  Lists and counts go round in threes: step k of a launch
+// group writes list k % 3, reads list (k - 1) % 3 and clears the count of
+// (k + 1) % 3; defer_flush_kernel delivers the group's last list.
+template <bool INT, bool XSYN, int BLOCK>
+__device__ __forceinline__ void deliver_listed(const EngineDev *__restrict__ eng, const NetDev &nd, uint32_t net,
+                                               uint32_t n_deliver, uint32_t k, uint32_t ts) {
+    const uint32_t lane = threadIdx.x & 31u, which = (k + 2u) % 3u;
+    const uint32_t w = blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5), nw = n_deliver * (BLOCK / 32);
+    const uint2 *list = reinterpret_cast<const uint2 *>(nd.slist) + (size_t)which * nd.n_pad;
+    uint2 row = make_uint2(0u, 0u);
+    if (w < nd.n_pad) row = list[w];  // with the count, not after it; used only below it
+    const uint32_t cnt = nd.scount[which];
+    if (w == 0u && lane == 0u) {
+        nd.scount[(k + 1u) % 3u] = 0u;
+        if (cnt) atomicAdd(&eng->counters[net].spikes_total, (unsigned long long)cnt);
+    }
+    const uint64_t pol = ring_policy();
+    for (uint32_t e = w; e < cnt; e += nw) {
+        const uint2 cur = row;
+        if (e + nw < cnt) row = list[e + nw];
+        defer_deliver<INT, XSYN>(nd, cur.x, cur.y - cur.x, ts, lane, false, pol);
+    }
+}
+
+template <bool INT, int BLOCK, bool ADEX, bool PLAIN>
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
+    step_kernel_defer(const EngineDev *__restrict__ eng, uint32_t n_deliver, uint32_t k_step) {
+    pdl_trigger();
+    __shared__ __align__(16) NetDev s_nd;
+    __shared__ __align__(16) ParamRow s_ptab[kSmemParamRows];
+    static_assert(sizeof(NetDev) / 16 <= BLOCK, "one 16-byte word per thread");
+    const bool deliver = blockIdx.x < n_deliver;
+    const Tile tile = eng->tiles[deliver ? 0u : blockIdx.x - n_deliver];
+    stage_net(eng, tile.net, &s_nd);
+    const ParamRow *ptab = deliver ? nullptr : stage_params<BLOCK>(eng, s_ptab);
+    __syncthreads();
+    pdl_wait();
+    const uint64_t t = s_nd.t + k_step;
+    uint32_t tmod = s_nd.tmod + k_step;
+    if (tmod >= s_nd.D) tmod %= s_nd.D;
+    if (deliver) {
+        if (k_step == 0u) return;  // nothing listed yet; the counts were cleared before the group
+        deliver_listed<INT, !PLAIN, BLOCK>(eng, s_nd, tile.net, n_deliver, k_step, tmod == 0u ? s_nd.D - 1u : tmod - 1u);
+        return;
+    }
+    const SmemLists none{};
+    process_tile<INT, BLOCK, 1, false, ADEX, false, PLAIN, PLAIN, false, true>(
+        eng, ptab, s_nd, tile, t, tmod, k_step, s_nd.v + tile.start, s_nd.u + tile.start, s_nd.s + tile.start,
+        s_nd.tk + tile.start, s_nd.pidx + tile.start, none);
+}
+
+// The last list of a launch group of `steps` steps.
+template <bool INT>
+__global__ void __launch_bounds__(128) defer_flush_kernel(const EngineDev *__restrict__ eng, uint32_t steps) {
+    pdl_trigger();
+    __shared__ __align__(16) NetDev s_nd;
+    const uint32_t net = eng->tiles[0].net;
+    stage_net(eng, net, &s_nd);
+    __syncthreads();
+    pdl_wait();
+    deliver_listed<INT, true, 128>(eng, s_nd, net, gridDim.x, steps, (s_nd.tmod + steps - 1u) % s_nd.D);
 }
 
 // ------------------------------------------- warp-specialised streaming kernel
@@ -1070,6 +1206,29 @@ cudaError_t StepKind<INT, ADEX>::launch(uint32_t block, uint32_t npt, int varian
     NE2B_SHAPES(X)
 #undef X
     return cudaErrorInvalidValue;
+}
+
+template <bool INT, bool ADEX>
+int StepKind<INT, ADEX>::defer_occupancy(bool plain) {
+    int b = 0;
+    if (plain)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, step_kernel_defer<INT, kDeferBlock, ADEX, true>, kDeferBlock, 0);
+    else
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, step_kernel_defer<INT, kDeferBlock, ADEX, false>, kDeferBlock, 0);
+    return b;
+}
+
+template <bool INT, bool ADEX>
+cudaError_t StepKind<INT, ADEX>::launch_defer(bool plain, const EngineDev *eng, uint32_t n_deliver, uint32_t k_step,
+                                              uint32_t grid, cudaStream_t st) {
+    return launch_pdl(plain ? step_kernel_defer<INT, kDeferBlock, ADEX, true> : step_kernel_defer<INT, kDeferBlock, ADEX, false>,
+                      grid, kDeferBlock, st, k_step > 0, eng, n_deliver, k_step);
+}
+
+template <bool INT, bool ADEX>
+cudaError_t StepKind<INT, ADEX>::launch_defer_flush(const EngineDev *eng, uint32_t n_deliver, uint32_t steps,
+                                                    cudaStream_t st) {
+    return launch_pdl(defer_flush_kernel<INT>, n_deliver, 128, st, true, eng, steps);
 }
 
 template <bool INT, bool ADEX>

@@ -38,6 +38,7 @@ __host__ __device__ constexpr uint32_t resident_head_bytes() {
 // optional ones (external current, stimulus, records, windows, custom-tau
 // synapses, f32 trace, watches), many nets (batches, the server), and many
 // nets without records, custom-tau synapses, f32 trace or watches.
+constexpr uint32_t kDeferBlock = 128;  // threads and neurons of a tile of step_kernel_defer
 enum StepVariant : int { kStepSingle = 0, kStepMulti = 1, kStepPlain = 2, kStepMultiLean = 3 };
 // Added to kStepSingle or kStepPlain: the warp-specialised instance
 // (separate delivery warps; engines of one net, NE2B_WS_SHAPES only).
@@ -60,6 +61,9 @@ inline uint32_t cluster_smem(uint32_t m, uint32_t hop, const ClusterShape &s) {
 
 template <bool INT, bool ADEX>
 struct StepKind {
+    static int defer_occupancy(bool plain);
+    static cudaError_t launch_defer(bool plain, const EngineDev *eng, uint32_t n_deliver, uint32_t k_step, uint32_t grid, cudaStream_t st);
+    static cudaError_t launch_defer_flush(const EngineDev *eng, uint32_t n_deliver, uint32_t steps, cudaStream_t st);
     // cluster kernel: `clusters` clusters of `blocks` blocks; `full` = with
     // records, custom-tau synapses, f32 trace and watches
     static int cluster_fit(bool full, uint32_t blocks, const ClusterShape &cs, size_t smem);

@@ -773,6 +773,7 @@ ne2b_status ne2b_server_create(const ne2b_server_config *cfg, int device, ne2b_s
                 return st;
             }
             b->sg.set_stream(b->st);
+            b->sg.set_min_block((size_t)64 << 20);
             ne2b_server::Builder *bp = b.get();
             s->builders.push_back(std::move(b));
             bp->th = std::thread(server_builder, s, bp);

@@ -321,8 +321,7 @@ ne2b_status Stager::reserve(size_t bytes, void **host) {
         }
         if (cur_ < 0) {
             PinnedBlock b;
-            // what this net needs, at least 4 MB: pinning costs 0.25 ms per MB
-            b.cap = std::max<size_t>(need, (size_t)4 << 20);
+            b.cap = std::max<size_t>(need, min_block_);
             NE2B_CUDA(cudaMallocHost(&b.p, b.cap));
             NE2B_CUDA(cudaEventCreateWithFlags(&b.ev, cudaEventDisableTiming));
             pin_.push_back(b);
@@ -640,27 +639,27 @@ ne2b_status Engine::build_net(const ne2b_net_desc *net, const ne2b_config *cfg, 
     }
     if (any_tau) {
         // XSyn::build (sim/src/state.rs:245-274): synapses with tau > 0 get
-        // their own current, numbered in CSR order; the neuron pass reads
-        // them grouped by target (CSR order within a target)
+        // their own current, numbered by target (CSR order within a target),
+        // so a neuron's are neighbours and a warp's are one range
         std::vector<uint32_t> xmap(h->e), xt_ptr((size_t)n + 1, 0);
-        uint32_t nx = 0;
-        for (uint64_t j = 0; j < h->e; ++j) xmap[j] = net->tau_ms[j] > 0.0f ? nx++ : kNoXsyn;
-        std::vector<float> xdecay(nx), xw(nx);
-        std::vector<uint32_t> xt_idx(nx);
-        for (uint64_t j = 0; j < h->e; ++j) {
-            const uint32_t k = xmap[j];
-            if (k == kNoXsyn) continue;
-            xdecay[k] = host_decay(cfg->dt_ms, net->tau_ms[j]);  // state.rs:262-264
-            // the arrival adds w; with the int ring it is rt_get(rt_put(w)),
-            // the value the fixed-point path delivers (kernels.rs:57-66)
-            xw[k] = int_ring_ ? (float)(int32_t)lrintf(net->w[j] * 4096.0f) / 4096.0f : net->w[j];
-            xt_ptr[net->tgt[j] + 1]++;
-        }
+        for (uint64_t j = 0; j < h->e; ++j)
+            if (net->tau_ms[j] > 0.0f) xt_ptr[net->tgt[j] + 1]++;
         for (uint32_t i = 0; i < n; ++i) xt_ptr[i + 1] += xt_ptr[i];
+        const uint32_t nx = xt_ptr[n];
+        std::vector<float> xdecay(nx), xw(nx);
         {
             std::vector<uint32_t> fill(xt_ptr.begin(), xt_ptr.end() - 1);
-            for (uint64_t j = 0; j < h->e; ++j)
-                if (xmap[j] != kNoXsyn) xt_idx[fill[net->tgt[j]]++] = xmap[j];
+            for (uint64_t j = 0; j < h->e; ++j) {
+                if (!(net->tau_ms[j] > 0.0f)) {
+                    xmap[j] = kNoXsyn;
+                    continue;
+                }
+                const uint32_t k = xmap[j] = fill[net->tgt[j]]++;
+                xdecay[k] = host_decay(cfg->dt_ms, net->tau_ms[j]);  // state.rs:262-264
+                // the arrival adds w; with the int ring it is rt_get(rt_put(w)),
+                // the value the fixed-point path delivers (kernels.rs:57-66)
+                xw[k] = int_ring_ ? (float)(int32_t)lrintf(net->w[j] * 4096.0f) / 4096.0f : net->w[j];
+            }
         }
         h->nx = nx;
         d.xwords = (nx + 31) / 32;
@@ -668,8 +667,6 @@ ne2b_status Engine::build_net(const ne2b_net_desc *net, const ne2b_config *cfg, 
         NET_TRY(up(p, xmap.data(), sizeof(uint32_t) * h->e));
         NET_TRY(alloc(&p, sizeof(uint32_t) * ((size_t)n + 1))); d.xt_ptr = (const uint32_t *)p;
         NET_TRY(up(p, xt_ptr.data(), sizeof(uint32_t) * ((size_t)n + 1)));
-        NET_TRY(alloc(&p, sizeof(uint32_t) * nx)); d.xt_idx = (const uint32_t *)p;
-        NET_TRY(up(p, xt_idx.data(), sizeof(uint32_t) * nx));
         NET_TRY(alloc(&p, sizeof(float) * nx)); d.xdecay = (const float *)p;
         NET_TRY(up(p, xdecay.data(), sizeof(float) * nx));
         NET_TRY(alloc(&p, sizeof(float) * nx)); d.xw = (const float *)p;
@@ -1069,8 +1066,8 @@ static uint32_t deliver_blocks(uint32_t n, int sm_count) {
 // 1.82 us, active 3.2 / 3.9; AdEx 2.20 / 2.23, 4.5 / 4.8; 20k 1.48 / 1.66, 2.6
 // / 3.2.  Past one wave it loses its point: the neuron pass takes longer than
 // the delivery it hides, and the fused kernel's larger tiles win (200k 2.8 /
-// 2.4, 5.8 / 5.3; 1M 8.9 / 6.4).  Not taken when more than one neuron in 16
-// has a synapse of delay 1: their rows would be read twice, a warp at a time.
+// 2.4, 5.8 / 5.3; 1M 8.9 / 6.4).  Not taken when more than one neuron in four
+// has a synapse of delay 1: their rows are read twice, a warp at a time.
 ne2b_status Engine::plan_defer() {
     if (mode_ != kModeAuto || shape_set_ || multi_net || active_nets() != 1) return NE2B_OK;
     NetHost *h = nullptr;
@@ -1079,7 +1076,7 @@ ne2b_status Engine::plan_defer() {
     if (!h->n) return NE2B_OK;
     defer_shape_.block = kDeferBlock;
     defer_shape_.npt = 1;
-    const uint32_t occ = (uint32_t)defer_occupancy(int_ring_, adex_, false);
+    const uint32_t occ = (uint32_t)defer_occupancy(int_ring_, adex_, h->nx ? kDeferXs : kDeferFull);
     if (h->n_pad / kDeferBlock + 1u + deliver_blocks(h->n, sm_count_) > occ * (uint32_t)sm_count_) return NE2B_OK;
     NetDev &d = h->dev;
     if (h->urgent < 0) {  // once per net
@@ -1098,7 +1095,7 @@ ne2b_status Engine::plan_defer() {
             h->urgent = (int64_t)count;
             d.urgent = bits;
         }
-        if (h->urgent * 16 <= (int64_t)h->n) {
+        if (h->urgent * 4 <= (int64_t)h->n) {
             NE2B_CUDA(cudaMallocAsync(&p, sizeof(uint2_pod) * 3 * (size_t)h->n_pad + 16, stream_));
             h->allocs.push_back(p);
             d.slist = (uint2_pod *)p;
@@ -1376,8 +1373,8 @@ ne2b_status Engine::launch_deferred(uint32_t steps) {
     NetHost *h = nullptr;
     for (NetHost *x : nets_)
         if (x) h = x;
-    const bool plain = step_variant(TileShape{}) == kStepPlain;
-    const int var = 0x100 | (plain ? 1 : 0);
+    const int inst = h->nx ? kDeferXs : step_variant(TileShape{}) == kStepPlain ? kDeferPlain : kDeferFull;
+    const int var = 0x100 | inst;
     if (var != graph_variant_) {
         clear_graphs();
         graph_variant_ = var;
@@ -1386,7 +1383,7 @@ ne2b_status Engine::launch_deferred(uint32_t steps) {
     auto group = [&]() -> cudaError_t {
         cudaError_t e = cudaMemsetAsync(h->dev.scount, 0, 3 * sizeof(uint32_t), stream_);
         for (uint32_t k = 0; k < steps && e == cudaSuccess; ++k)
-            e = launch_defer(int_ring_, adex_, plain, d_eng_, nd, k, grid, stream_);
+            e = launch_defer(int_ring_, adex_, inst, d_eng_, nd, k, grid, stream_);
         if (e == cudaSuccess) e = launch_defer_flush(int_ring_, adex_, d_eng_, nd, steps, stream_);
         if (e == cudaSuccess) e = launch_advance(d_nets_, nets_cap_, steps, stream_);
         return e;

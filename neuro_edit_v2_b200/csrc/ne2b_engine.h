@@ -116,6 +116,10 @@ class Stager {
     Stager &operator=(const Stager &) = delete;
     ~Stager();
     void set_stream(cudaStream_t st) { st_ = st; }
+    // Smallest pinned block.  Pinning costs 0.25 ms per MB, so a sim pins
+    // what its net needs; an admission thread stages one request after
+    // another of different sizes and keeps blocks that fit most of them.
+    void set_min_block(size_t bytes) { min_block_ = bytes; }
     cudaStream_t stream() const { return st_; }
     ne2b_status reserve(size_t bytes, void **host);
     ne2b_status issue(void *dst, const void *host, size_t bytes);
@@ -139,6 +143,7 @@ class Stager {
     int ring_next_ = 0;
     cudaStream_t st_ = nullptr;
     std::vector<PinnedBlock> pin_;
+    size_t min_block_ = (size_t)4 << 20;
     int cur_ = -1;
     std::vector<int> open_;
 };

@@ -29,8 +29,8 @@ cudaError_t launch_resident(bool int_ring, bool adex, uint32_t block, uint32_t n
                             uint32_t k0, uint32_t nsteps, uint32_t grid, size_t smem, cudaStream_t st);
 // Deferred-delivery kernel (step_kernel_defer): `grid` blocks, the first
 // `n_deliver` of which deliver; after a group's steps, the flush.
-int defer_occupancy(bool int_ring, bool adex, bool plain);
-cudaError_t launch_defer(bool int_ring, bool adex, bool plain, const EngineDev *eng, uint32_t n_deliver,
+int defer_occupancy(bool int_ring, bool adex, int variant);
+cudaError_t launch_defer(bool int_ring, bool adex, int variant, const EngineDev *eng, uint32_t n_deliver,
                          uint32_t k_step, uint32_t grid, cudaStream_t st);
 cudaError_t launch_defer_flush(bool int_ring, bool adex, const EngineDev *eng, uint32_t n_deliver, uint32_t steps,
                                cudaStream_t st);

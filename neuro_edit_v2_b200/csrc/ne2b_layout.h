@@ -109,8 +109,7 @@ struct alignas(16) NetDev {
     uint16_t *win_out;      // [max_windows x n_pad]
     // synapses with their own tau (sim/src/state.rs:231-275), kNetXsyn only
     const uint32_t *xmap;   // [E] custom-synapse id of CSR synapse j, or kNoXsyn
-    const uint32_t *xt_ptr; // [n+1] each target's range in xt_idx
-    const uint32_t *xt_idx; // [nx] custom-synapse ids grouped by target, CSR order within
+    const uint32_t *xt_ptr; // [n+1] each target's range of custom-synapse ids (CSR order within)
     float *xsyn;            // [nx] each custom synapse's current
     const float *xdecay;    // [nx] exp(-dt / tau)
     const float *xw;        // [nx] arrival weight (rt_get(rt_put(w)) with the int ring)

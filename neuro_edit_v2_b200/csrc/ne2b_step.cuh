@@ -177,18 +177,70 @@ __device__ __forceinline__ void defer_deliver(const NetDev &nd, uint32_t rlo, ui
     }
 }
 
+// Synapses with their own tau (cpu.rs:206-228): an arrival due this step (its
+// bit in this slot's words) adds w, then the current joins the target's input
+// and decays; a synapse arrives at most once per step, so arrivals commute
+// and fold into this pass.  The currents of a warp's 32 targets are one range
+// of ids: the lanes stride it, 256 ids at a time, every load coalesced and in
+// flight together, and leave the currents in shared memory, from which each
+// lane adds its own neuron's in order.  (A lane walking its own list, one id
+// after another with five dependent scattered loads each, took 41 us per step
+// on 20k neurons with 10 custom synapses each; so 10.8 us, and 6.5 with
+// delivery deferred.)
+constexpr uint32_t kXChunk = 256;
+template <bool RES>
+__device__ __forceinline__ void custom_currents(const NetDev &nd, uint32_t tmod, uint32_t p0, uint32_t p1, bool valid,
+                                                float &I, float *xs, uint32_t lane) {
+    // valid lanes are the first ones of the warp (none in a warp past the net)
+    const uint32_t live = __ballot_sync(0xffffffffu, valid);
+    if (live == 0u) return;
+    const uint32_t lo = __shfl_sync(0xffffffffu, p0, 0), hi = __shfl_sync(0xffffffffu, p1, 31 - __clz(live));
+    uint32_t *pend = nd.xpend + (size_t)tmod * nd.xwords;
+    for (uint32_t base = lo; base < hi; base += kXChunk) {
+        const uint32_t m = min(kXChunk, hi - base);
+        float x[kXChunk / 32], dec[kXChunk / 32];
+        uint32_t word[kXChunk / 32];
+#pragma unroll
+        for (uint32_t e = 0; e < kXChunk / 32; ++e) {
+            const uint32_t k = base + e * 32u + lane;
+            x[e] = dec[e] = 0.0f;
+            word[e] = 0u;
+            if (e * 32u + lane < m) {
+                x[e] = nd.xsyn[k];
+                dec[e] = nd.xdecay[k];
+                word[e] = RES ? __ldcg(pend + (k >> 5)) : pend[k >> 5];
+            }
+        }
+#pragma unroll
+        for (uint32_t e = 0; e < kXChunk / 32; ++e) {
+            const uint32_t k = base + e * 32u + lane, bit = 1u << (k & 31u);
+            if (e * 32u + lane >= m) continue;
+            if (word[e] & bit) {
+                x[e] = __fadd_rn(x[e], nd.xw[k]);
+                atomicAnd(pend + (k >> 5), ~bit);  // other bits of the word belong to other targets
+            }
+            xs[e * 32u + lane] = x[e];
+            nd.xsyn[k] = __fmul_rn(x[e], dec[e]);
+        }
+        __syncwarp();
+        for (uint32_t j = max(p0, base); j < min(p1, base + m); ++j) I = __fadd_rn(I, xs[j - base]);
+        __syncwarp();
+    }
+}
+
 // WSQ (step_kernel_ws): the tile's threads are the producer warps of a
 // delivery queue; they push their spiking neurons' rows into `wq` and count
 // their spikes into *nspk (per warp) instead of compacting and delivering.
 // DEFER (step_kernel_defer): each warp appends its spiking neurons' rows to
 // the step's spike list, which the next step's delivery blocks take, and
-// delivers at once only synapses of delay 1.
+// delivers at once only synapses of delay 1.  XS: custom-tau synapses compiled
+// in (with !LEAN).
 template <bool INT, int BLOCK, int NPT, bool RES, bool ADEX, bool PHASES, bool LEAN = false, bool NOIO = false,
-          bool WSQ = false, bool DEFER = false>
+          bool WSQ = false, bool DEFER = false, bool XS = true>
 __device__ __forceinline__ void process_tile(const EngineDev *__restrict__ eng, const ParamRow *ptab, const NetDev &nd,
                                              const Tile &tile, uint64_t t, uint32_t tmod, uint32_t k, float *vs, float *us,
                                              float *ss, uint16_t *tks, const uint16_t *pis, const SmemLists &sl,
-                                             const WsQueue *wq = nullptr, uint32_t *nspk = nullptr) {
+                                             float *xbuf, const WsQueue *wq = nullptr, uint32_t *nspk = nullptr) {
     constexpr int NW = BLOCK / 32;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -207,7 +259,7 @@ __device__ __forceinline__ void process_tile(const EngineDev *__restrict__ eng, 
     const bool has_ext = !NOIO && (flags & kNetHasExt);
     const bool has_stim = !NOIO && (tile.flags & kTileHasStim);
     const bool windows = !NOIO && (flags & kNetWindows);
-    const bool xsyn_on = !LEAN && (flags & kNetXsyn);
+    const bool xsyn_on = !LEAN && XS && (flags & kNetXsyn);
     bool win_end = false;
     uint32_t widx = 0;
     if (windows) {
@@ -229,6 +281,7 @@ __device__ __forceinline__ void process_tile(const EngineDev *__restrict__ eng, 
     bool valid[NPT];
     float v[NPT], u[NPT], s[NPT], ex[NPT];
     uint32_t rw[NPT], tk[NPT], pi[NPT];
+    uint32_t xp0[NPT], xp1[NPT];  // the neuron's custom synapses, loaded with its state
 #pragma unroll
     for (int q = 0; q < NPT; ++q) {
         const uint32_t off = q * BLOCK + threadIdx.x;
@@ -242,6 +295,11 @@ __device__ __forceinline__ void process_tile(const EngineDev *__restrict__ eng, 
             tk[q] = tks[off];
             pi[q] = pis[off];
             ex[q] = has_ext ? nd.ext[li[q]] : 0.0f;
+        }
+        xp0[q] = xp1[q] = 0u;
+        if (xsyn_on && valid[q]) {
+            xp0[q] = nd.xt_ptr[li[q]];
+            xp1[q] = nd.xt_ptr[li[q] + 1];
         }
     }
     // warm L2 with the next step's ring slot (one prefetch per 32-byte
@@ -270,32 +328,20 @@ __device__ __forceinline__ void process_tile(const EngineDev *__restrict__ eng, 
     for (int q = 0; q < NPT; ++q) {
         spk[q] = false;
         rlo[q] = rhi[q] = 0u;
-        if (!valid[q]) continue;
+        if (!xsyn_on && !valid[q]) continue;
         const uint32_t i = li[q];
         const uint32_t off = q * BLOCK + threadIdx.x;
-        const float arr = INT ? __fmul_rn(__int2float_rn((int)rw[q]), 0x1p-12f)  // rt_get, kernels.rs:60
-                              : __uint_as_float(rw[q]);
-        if (rw[q] != 0u) ringw[slot_off + i] = 0u;
-        const float sv = __fadd_rn(s[q], arr);
-        float I = __fadd_rn(sv, ex[q]);
+        float sv = 0.0f, I = 0.0f;
+        if (LEAN || !XS || valid[q]) {
+            const float arr = INT ? __fmul_rn(__int2float_rn((int)rw[q]), 0x1p-12f)  // rt_get, kernels.rs:60
+                                  : __uint_as_float(rw[q]);
+            if (rw[q] != 0u) ringw[slot_off + i] = 0u;
+            sv = __fadd_rn(s[q], arr);
+            I = __fadd_rn(sv, ex[q]);
+        }
         if (xsyn_on) {
-            // synapses with their own tau (cpu.rs:206-228): an arrival due
-            // this step (its bit in this slot's words) adds w, then the
-            // current joins the input and decays; a synapse arrives at most
-            // once per step, so arrivals commute and fold into this loop
-            uint32_t *pend = nd.xpend + (size_t)tmod * nd.xwords;
-            for (uint32_t j = nd.xt_ptr[i], je = nd.xt_ptr[i + 1]; j < je; ++j) {
-                const uint32_t k = nd.xt_idx[j];
-                const uint32_t bit = 1u << (k & 31u);
-                float x = nd.xsyn[k];
-                const uint32_t word = RES ? __ldcg(pend + (k >> 5)) : pend[k >> 5];
-                if (word & bit) {
-                    x = __fadd_rn(x, nd.xw[k]);
-                    atomicAnd(pend + (k >> 5), ~bit);  // other bits of the word belong to other targets
-                }
-                I = __fadd_rn(I, x);
-                nd.xsyn[k] = __fmul_rn(x, nd.xdecay[k]);
-            }
+            custom_currents<RES>(nd, tmod, xp0[q], xp1[q], valid[q], I, xbuf + warp * kXChunk, lane);
+            if (!valid[q]) continue;
         }
         if (has_stim) {
             // the host provides the [steps x inputs] values covering every
@@ -411,7 +457,7 @@ __device__ __forceinline__ void process_tile(const EngineDev *__restrict__ eng, 
             for (uint32_t u = urg; u; u &= u - 1u) {  // rare: the row's synapses of delay 1, now
                 const int l = __ffs(u) - 1;
                 const uint32_t lo = __shfl_sync(0xffffffffu, rlo[q], l), hi = __shfl_sync(0xffffffffu, rhi[q], l);
-                defer_deliver<INT, !LEAN>(nd, lo, hi - lo, tmod, lane, true, ring_policy());
+                defer_deliver<INT, !LEAN && XS>(nd, lo, hi - lo, tmod, lane, true, ring_policy());
             }
         }
         return;
@@ -639,6 +685,7 @@ __device__ __forceinline__ void step_body(const EngineDev *__restrict__ eng, uin
     __shared__ uint32_t s_lists[smem_lists_words<BLOCK, NPT>()];
     __shared__ __align__(16) NetDev s_nd;
     __shared__ __align__(16) ParamRow s_ptab[kSmemParamRows];
+    __shared__ float s_x[PLAIN ? 1 : BLOCK / 32 * kXChunk];
     static_assert(sizeof(NetDev) % 16 == 0 && sizeof(ParamRow) % 16 == 0, "16-byte staging");
     static_assert(kNetWords <= BLOCK && kStageTiles <= BLOCK, "one 16-byte word per thread");
     const SmemLists sl = smem_lists(s_lists, BLOCK * NPT, BLOCK / 32);
@@ -659,7 +706,7 @@ __device__ __forceinline__ void step_body(const EngineDev *__restrict__ eng, uin
             process_tile<INT, BLOCK, NPT, false, ADEX, false, PLAIN, PLAIN>(eng, ptab, s_nd, tile, t, tmod, k_step,
                                                              s_nd.v + tile.start, s_nd.u + tile.start,
                                                              s_nd.s + tile.start, s_nd.tk + tile.start,
-                                                             s_nd.pidx + tile.start, sl);
+                                                             s_nd.pidx + tile.start, sl, s_x);
             if (nx >= n_tiles) break;
             const Tile next = eng->tiles[nx];
             if (next.net != tile.net) {
@@ -710,7 +757,7 @@ __device__ __forceinline__ void step_body(const EngineDev *__restrict__ eng, uin
             process_tile<INT, BLOCK, NPT, false, ADEX, true, PLAIN>(eng, ptab, s_nd, tile, t, tmod, k_step,
                                                             s_nd.v + tile.start, s_nd.u + tile.start,
                                                             s_nd.s + tile.start, s_nd.tk + tile.start,
-                                                            s_nd.pidx + tile.start, sl);
+                                                            s_nd.pidx + tile.start, sl, s_x);
         }
     }
 }
@@ -766,12 +813,15 @@ __device__ __forceinline__ void deliver_listed(const EngineDev *__restrict__ eng
     }
 }
 
-template <bool INT, int BLOCK, bool ADEX, bool PLAIN>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
+// XS: the net has custom-tau synapses, whose pass needs more than the 64
+// registers that let eight blocks share an SM.
+template <bool INT, int BLOCK, bool ADEX, bool PLAIN, bool XS>
+__global__ void __launch_bounds__(BLOCK, (XS ? 512 : 1024) / BLOCK)
     step_kernel_defer(const EngineDev *__restrict__ eng, uint32_t n_deliver, uint32_t k_step) {
     pdl_trigger();
     __shared__ __align__(16) NetDev s_nd;
     __shared__ __align__(16) ParamRow s_ptab[kSmemParamRows];
+    __shared__ float s_x[XS ? BLOCK / 32 * kXChunk : 1];
     static_assert(sizeof(NetDev) / 16 <= BLOCK, "one 16-byte word per thread");
     const bool deliver = blockIdx.x < n_deliver;
     const Tile tile = eng->tiles[deliver ? 0u : blockIdx.x - n_deliver];
@@ -784,13 +834,13 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
     if (tmod >= s_nd.D) tmod %= s_nd.D;
     if (deliver) {
         if (k_step == 0u) return;  // nothing listed yet; the counts were cleared before the group
-        deliver_listed<INT, !PLAIN, BLOCK>(eng, s_nd, tile.net, n_deliver, k_step, tmod == 0u ? s_nd.D - 1u : tmod - 1u);
+        deliver_listed<INT, XS, BLOCK>(eng, s_nd, tile.net, n_deliver, k_step, tmod == 0u ? s_nd.D - 1u : tmod - 1u);
         return;
     }
     const SmemLists none{};
-    process_tile<INT, BLOCK, 1, false, ADEX, false, PLAIN, PLAIN, false, true>(
+    process_tile<INT, BLOCK, 1, false, ADEX, false, PLAIN, PLAIN, false, true, XS>(
         eng, ptab, s_nd, tile, t, tmod, k_step, s_nd.v + tile.start, s_nd.u + tile.start, s_nd.s + tile.start,
-        s_nd.tk + tile.start, s_nd.pidx + tile.start, none);
+        s_nd.tk + tile.start, s_nd.pidx + tile.start, none, s_x);
 }
 
 // The last list of a launch group of `steps` steps.
@@ -830,6 +880,7 @@ __global__ void __launch_bounds__(BLOCK + 32 * ws_warps<BLOCK>()) step_kernel_ws
     __shared__ __align__(16) NetDev s_nd;
     __shared__ __align__(16) ParamRow s_ptab[kSmemParamRows];
     __shared__ __align__(16) uint4 s_cell[kWsCells];
+    __shared__ float s_x[PLAIN ? 1 : BLOCK / 32 * kXChunk];
     __shared__ uint32_t s_ctr[4];
     static_assert(sizeof(NetDev) / 16 <= BLOCK, "one 16-byte word per thread");
     const uint32_t n_tiles = eng->n_tiles;
@@ -853,7 +904,7 @@ __global__ void __launch_bounds__(BLOCK + 32 * ws_warps<BLOCK>()) step_kernel_ws
         for (;;) {
             process_tile<INT, BLOCK, NPT, false, ADEX, false, PLAIN, PLAIN, true>(
                 eng, ptab, s_nd, tile, t, tmod, k_step, s_nd.v + tile.start, s_nd.u + tile.start, s_nd.s + tile.start,
-                s_nd.tk + tile.start, s_nd.pidx + tile.start, none, &wq, &nspk);
+                s_nd.tk + tile.start, s_nd.pidx + tile.start, none, s_x, &wq, &nspk);
             tix += gridDim.x;
             if (tix >= n_tiles) break;
             tile = eng->tiles[tix];
@@ -1018,6 +1069,7 @@ __global__ void __launch_bounds__(BLOCK) resident_kernel(const EngineDev *__rest
     uint16_t *stk = reinterpret_cast<uint16_t *>(ss + M);
     uint16_t *spi = stk + M;
     __shared__ __align__(16) ParamRow s_ptab[kSmemParamRows];
+    __shared__ float s_x[BLOCK / 32 * kXChunk];
     const ParamRow *ptab = stage_params<BLOCK>(eng, s_ptab);
     const uint32_t t_lo = eng->block_tiles[blockIdx.x], t_hi = eng->block_tiles[blockIdx.x + 1];
 
@@ -1044,7 +1096,7 @@ __global__ void __launch_bounds__(BLOCK) resident_kernel(const EngineDev *__rest
             uint32_t tmod = nd.tmod + k0 + k;
             if (tmod >= nd.D) tmod %= nd.D;
             process_tile<INT, BLOCK, NPT, true, ADEX, false>(eng, ptab, nd, tile, t, tmod, k0 + k, sv + o, su + o,
-                                                             ss + o, stk + o, spi + o, sl);
+                                                             ss + o, stk + o, spi + o, sl, s_x);
         }
         if (k + 1 < nsteps && !grid_barrier(eng->barrier, (k + 1) * gridDim.x, eng->err, s_flag)) break;
     }
@@ -1209,20 +1261,23 @@ cudaError_t StepKind<INT, ADEX>::launch(uint32_t block, uint32_t npt, int varian
 }
 
 template <bool INT, bool ADEX>
-int StepKind<INT, ADEX>::defer_occupancy(bool plain) {
+static auto defer_instance(int variant) {
+    return variant == kDeferPlain ? step_kernel_defer<INT, kDeferBlock, ADEX, true, false>
+           : variant == kDeferXs  ? step_kernel_defer<INT, kDeferBlock, ADEX, false, true>
+                                  : step_kernel_defer<INT, kDeferBlock, ADEX, false, false>;
+}
+
+template <bool INT, bool ADEX>
+int StepKind<INT, ADEX>::defer_occupancy(int variant) {
     int b = 0;
-    if (plain)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, step_kernel_defer<INT, kDeferBlock, ADEX, true>, kDeferBlock, 0);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, step_kernel_defer<INT, kDeferBlock, ADEX, false>, kDeferBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, defer_instance<INT, ADEX>(variant), kDeferBlock, 0);
     return b;
 }
 
 template <bool INT, bool ADEX>
-cudaError_t StepKind<INT, ADEX>::launch_defer(bool plain, const EngineDev *eng, uint32_t n_deliver, uint32_t k_step,
+cudaError_t StepKind<INT, ADEX>::launch_defer(int variant, const EngineDev *eng, uint32_t n_deliver, uint32_t k_step,
                                               uint32_t grid, cudaStream_t st) {
-    return launch_pdl(plain ? step_kernel_defer<INT, kDeferBlock, ADEX, true> : step_kernel_defer<INT, kDeferBlock, ADEX, false>,
-                      grid, kDeferBlock, st, k_step > 0, eng, n_deliver, k_step);
+    return launch_pdl(defer_instance<INT, ADEX>(variant), grid, kDeferBlock, st, k_step > 0, eng, n_deliver, k_step);
 }
 
 template <bool INT, bool ADEX>

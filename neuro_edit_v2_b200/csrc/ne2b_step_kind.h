@@ -39,6 +39,9 @@ __host__ __device__ constexpr uint32_t resident_head_bytes() {
 // synapses, f32 trace, watches), many nets (batches, the server), and many
 // nets without records, custom-tau synapses, f32 trace or watches.
 constexpr uint32_t kDeferBlock = 128;  // threads and neurons of a tile of step_kernel_defer
+// Its instances: without the optional features, with them, and with custom-tau
+// synapses as well.
+enum DeferVariant : int { kDeferPlain = 0, kDeferFull = 1, kDeferXs = 2 };
 enum StepVariant : int { kStepSingle = 0, kStepMulti = 1, kStepPlain = 2, kStepMultiLean = 3 };
 // Added to kStepSingle or kStepPlain: the warp-specialised instance
 // (separate delivery warps; engines of one net, NE2B_WS_SHAPES only).
@@ -61,8 +64,8 @@ inline uint32_t cluster_smem(uint32_t m, uint32_t hop, const ClusterShape &s) {
 
 template <bool INT, bool ADEX>
 struct StepKind {
-    static int defer_occupancy(bool plain);
-    static cudaError_t launch_defer(bool plain, const EngineDev *eng, uint32_t n_deliver, uint32_t k_step, uint32_t grid, cudaStream_t st);
+    static int defer_occupancy(int variant);
+    static cudaError_t launch_defer(int variant, const EngineDev *eng, uint32_t n_deliver, uint32_t k_step, uint32_t grid, cudaStream_t st);
     static cudaError_t launch_defer_flush(const EngineDev *eng, uint32_t n_deliver, uint32_t steps, cudaStream_t st);
     // cluster kernel: `clusters` clusters of `blocks` blocks; `full` = with
     // records, custom-tau synapses, f32 trace and watches

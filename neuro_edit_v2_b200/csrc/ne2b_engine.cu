@@ -94,6 +94,7 @@ Engine::~Engine() {
     }
     if (stream_) cudaStreamSynchronize(stream_);
     if (stage_) cudaFreeHost(stage_);
+    if (fetch_pin_) cudaFreeHost(fetch_pin_);
     cudaFree(d_nets_);
     cudaFree(d_counters_);
     cudaFree(d_ptab_);
@@ -381,6 +382,10 @@ void Engine::discard_net(NetHost *h, cudaStream_t st) {
 }
 
 ne2b_status Engine::attach_net(NetHost *h, uint32_t *slot_out, bool rebuild) {
+    if (!fixed_grid) {  // pinned with the net, not by the first read of its state (the server's results go another way)
+        std::lock_guard<std::mutex> lk(fetch_mu_);
+        NE2B_TRY(fetch_reserve(64 + std::min(kFetchPinned, sizeof(float) * (size_t)h->n)));
+    }
     uint32_t slot = nets_cap_;
     for (uint32_t j = 0; j < nets_cap_; ++j)
         if (!nets_[j]) {
@@ -1223,9 +1228,44 @@ ne2b_status Engine::reset_net(uint32_t slot) {
     return upload_net(h);
 }
 
-ne2b_status Engine::sync() {
+ne2b_status Engine::sync() { return fetch(nullptr, nullptr, 0, true); }
+
+// The pinned buffer of fetch, at least `bytes` (with fetch_mu_ held).
+ne2b_status Engine::fetch_reserve(size_t bytes) {
+    if (fetch_cap_ >= bytes) return NE2B_OK;
+    size_t cap = (size_t)64 << 10;
+    while (cap < bytes) cap *= 2;
+    if (fetch_pin_) cudaFreeHost(fetch_pin_);
+    fetch_pin_ = nullptr;
+    fetch_cap_ = 0;
+    NE2B_CUDA(cudaMallocHost(&fetch_pin_, cap));
+    fetch_cap_ = cap;
+    return NE2B_OK;
+}
+
+// Device memory to the caller's buffer, after everything queued; `check`
+// reports a device wait that gave up since the last check.  Small reads go
+// through a pinned buffer, the error flag beside them under the same
+// synchronisation: a pageable copy of 4 KB and a second, blocking one of the
+// flag took 29 us, this takes 13.  Larger reads, and those that find the
+// buffer in another thread's hands, copy straight to the pageable buffer.
+ne2b_status Engine::fetch(void *out, const void *dev, size_t bytes, bool check) {
+    constexpr size_t kFlag = 64;  // the flag's place, before the data
+    std::unique_lock<std::mutex> lk(fetch_mu_, std::try_to_lock);
+    if (lk.owns_lock() && bytes <= kFetchPinned) {
+        NE2B_TRY(fetch_reserve(kFlag + bytes));
+        uint8_t *pin = (uint8_t *)fetch_pin_;
+        if (bytes) NE2B_CUDA(cudaMemcpyAsync(pin + kFlag, dev, bytes, cudaMemcpyDeviceToHost, stream_));
+        if (check) NE2B_CUDA(cudaMemcpyAsync(pin, d_err_, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream_));
+        NE2B_CUDA(cudaStreamSynchronize(stream_));
+        if (bytes) memcpy(out, pin + kFlag, bytes);
+        unsigned int e = 0;
+        if (check) memcpy(&e, pin, sizeof e);
+        return e ? check_err() : NE2B_OK;
+    }
+    if (bytes) NE2B_CUDA(cudaMemcpyAsync(out, dev, bytes, cudaMemcpyDeviceToHost, stream_));
     NE2B_CUDA(cudaStreamSynchronize(stream_));
-    return check_err();
+    return check ? check_err() : NE2B_OK;
 }
 
 // A grid barrier of the resident kernel that timed out leaves a flag; the
@@ -1472,9 +1512,7 @@ ne2b_status Engine::read_csr(NetHost &h, uint32_t *rowptr, uint32_t *tgt, uint32
 
 ne2b_status Engine::read_f32(const float *dev, uint32_t n, float *out) {
     if (n == 0) return NE2B_OK;
-    NE2B_CUDA(cudaMemcpyAsync(out, dev, sizeof(float) * n, cudaMemcpyDeviceToHost, stream_));
-    NE2B_CUDA(cudaStreamSynchronize(stream_));
-    return check_err();
+    return fetch(out, dev, sizeof(float) * n, true);
 }
 
 ne2b_status Engine::read_trace(NetHost &h, float *out) {
@@ -1484,11 +1522,10 @@ ne2b_status Engine::read_trace(NetHost &h, float *out) {
     NE2B_CUDA(cudaMallocAsync((void **)&tmp, sizeof(float) * h.n, stream_));
     cudaError_t e = launch_trace(h.dev.tk, h.dev.trace_tab, h.n, tmp, stream_);
     launches_ += 1;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out, tmp, sizeof(float) * h.n, cudaMemcpyDeviceToHost, stream_);
+    ne2b_status st = cuda_error(e, "trace readback");
+    if (st == NE2B_OK) st = fetch(out, tmp, sizeof(float) * h.n, true);
     cudaFreeAsync(tmp, stream_);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
-    NE2B_TRY(cuda_error(e, "trace readback"));
-    return check_err();
+    return st;
 }
 
 ne2b_status Engine::spike_counts(NetHost &h, uint64_t rows, uint32_t *out) {
@@ -1507,10 +1544,10 @@ ne2b_status Engine::spike_counts(NetHost &h, uint64_t rows, uint32_t *out) {
     if (rows >= h.t) e = launch_pn_total(h.dev.pn_total, n, tmp, stream_);
     else e = launch_window_count(h.dev.rec_bits, h.dev.rec_rows, h.n_pad, n, h.t, (uint32_t)rows, tmp, stream_);
     launches_ += 1;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out, tmp, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, stream_);
+    ne2b_status st = cuda_error(e, "spike_counts");
+    if (st == NE2B_OK) st = fetch(out, tmp, sizeof(uint32_t) * n, false);
     cudaFreeAsync(tmp, stream_);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
-    return cuda_error(e, "spike_counts");
+    return st;
 }
 
 ne2b_status Engine::spike_row(NetHost &h, uint32_t back, uint64_t *out) {
@@ -1520,26 +1557,18 @@ ne2b_status Engine::spike_row(NetHost &h, uint32_t back, uint64_t *out) {
     const uint64_t t = h.t - 1 - back;
     const uint32_t row = (uint32_t)(t % rr);
     const uint32_t words = (h.n + 63) / 64;
-    NE2B_CUDA(cudaMemcpyAsync(out, h.dev.rec_bits + (size_t)row * (h.n_pad / 32), sizeof(uint64_t) * words,
-                              cudaMemcpyDeviceToHost, stream_));
-    NE2B_CUDA(cudaStreamSynchronize(stream_));
-    return NE2B_OK;
+    return fetch(out, h.dev.rec_bits + (size_t)row * (h.n_pad / 32), sizeof(uint64_t) * words, false);
 }
 
 ne2b_status Engine::spikes_total(NetHost &h, uint64_t *out) {
-    NE2B_CUDA(cudaMemcpyAsync(out, &d_counters_[h.slot].spikes_total, sizeof(uint64_t), cudaMemcpyDeviceToHost, stream_));
-    NE2B_CUDA(cudaStreamSynchronize(stream_));
-    return NE2B_OK;
+    return fetch(out, &d_counters_[h.slot].spikes_total, sizeof(uint64_t), false);
 }
 
 ne2b_status Engine::window_counts(NetHost &h, uint32_t window, uint16_t *out) {
     if (!h.dev.win_out) return set_error(NE2B_EINVAL, "window counts are off (window_steps = 0)");
     if (window >= h.dev.max_windows) return set_error(NE2B_EINVAL, "window %u >= max_windows %u", window, h.dev.max_windows);
     if (h.n == 0) return NE2B_OK;
-    NE2B_CUDA(cudaMemcpyAsync(out, h.dev.win_out + (size_t)window * h.n_pad, sizeof(uint16_t) * h.n,
-                              cudaMemcpyDeviceToHost, stream_));
-    NE2B_CUDA(cudaStreamSynchronize(stream_));
-    return NE2B_OK;
+    return fetch(out, h.dev.win_out + (size_t)window * h.n_pad, sizeof(uint16_t) * h.n, false);
 }
 
 ne2b_status Engine::set_ext(NetHost &h, const float *ext, uint32_t len) {

@@ -198,6 +198,8 @@ class Engine {
     ne2b_status read_f32(const float *dev, uint32_t n, float *out);
     ne2b_status read_trace(NetHost &h, float *out);
     ne2b_status check_err();
+    ne2b_status fetch_reserve(size_t bytes);
+    ne2b_status fetch(void *out, const void *dev, size_t bytes, bool check);
     ne2b_status spike_counts(NetHost &h, uint64_t rows, uint32_t *out);
     ne2b_status spike_row(NetHost &h, uint32_t back, uint64_t *out);
     ne2b_status spikes_total(NetHost &h, uint64_t *out);
@@ -317,6 +319,10 @@ class Engine {
     unsigned int *d_err_ = nullptr;
     Stager stager_;  // uploads on the engine's own stream
     std::mutex ptab_mu_;  // the parameter dictionary (builds may run on other threads)
+    static constexpr size_t kFetchPinned = (size_t)512 << 10;  // reads up to this size are staged
+    std::mutex fetch_mu_;
+    void *fetch_pin_ = nullptr;
+    size_t fetch_cap_ = 0;
     void *stage_ = nullptr;  // pinned staging for stimulus chunks and descriptors
     size_t stage_bytes_ = 0;
 };

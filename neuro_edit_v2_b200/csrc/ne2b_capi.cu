@@ -143,7 +143,7 @@ static ne2b_status create_from_list(ne2b::Engine &eng, const ne2b_net_desc *net,
     if (d_dly) dc.syn.delay_ms = dly; else { LIST_TRY(dalloc(4 * E, &p)); dc.syn.delay_ms = (const float *)p; }
     if (d_kind) dc.syn.kind = kind; else { LIST_TRY(dalloc(n, &p)); dc.syn.kind = (const uint8_t *)p; }
     LIST_TRY(dalloc(2 * E, &p)); dc.steps = (const uint16_t *)p;
-    LIST_TRY(dalloc(4 * E, &p)); dc.place = (const uint32_t *)p;
+    if (csr_list_short(E)) { LIST_TRY(dalloc(4 * E, &p)); dc.place = (const uint32_t *)p; }
     LIST_TRY(dalloc(4 * (size_t)n, &p)); dc.counts = (const uint32_t *)p;
     LIST_TRY(dalloc(4 * (size_t)n, &p)); dc.cursor = (uint32_t *)p;
     LIST_TRY(dalloc(4 * (size_t)csr_scan_blocks(n), &p)); dc.sums = (uint32_t *)p;
@@ -184,7 +184,7 @@ static ne2b_status create_from_list(ne2b::Engine &eng, const ne2b_net_desc *net,
     }
     dc.max_delay = sc.max_delay;
     dc.min_delay = sc.min_delay;
-    dc.short_rows = csr_rows_short(sc.max_row);
+    dc.short_rows = dc.place && csr_rows_short(sc.max_row);
     LIST_TRY(eng.add_net_device_csr(net, cfg, dc, slot));
     LIST_TRY(cuda_error(cudaMemcpyAsync(&sc, dc.sc, sizeof sc, cudaMemcpyDeviceToHost, st), "scatter readback"));
     LIST_TRY(cuda_error(cudaStreamSynchronize(st), "device CSR build"));
@@ -478,9 +478,12 @@ ne2b_status ne2b_set_delivery_warps(ne2b_sim *sim, int32_t on) {
 
 ne2b_status ne2b_delivery_warps(ne2b_sim *sim, int32_t *on, int32_t *active) {
     if (!sim || !on || !active) return set_error(NE2B_EINVAL, "null argument");
-    *on = sim->eng.shape().ws ? 1 : 0;
-    *active = (!sim->eng.resident() && !sim->eng.cluster() && !sim->eng.deferred() && sim->eng.ws_applies(sim->eng.shape())) ? 1 : 0;
-    return NE2B_OK;
+    GUARD(([&]() -> ne2b_status {
+        *on = sim->eng.shape().ws ? 1 : 0;
+        *active = (!sim->eng.resident() && !sim->eng.cluster() && !sim->eng.deferred() &&
+                   sim->eng.ws_applies(sim->eng.shape())) ? 1 : 0;
+        return NE2B_OK;
+    })());
 }
 
 ne2b_status ne2b_stream(ne2b_sim *sim, void **stream) {

@@ -91,7 +91,7 @@ __global__ void csr_prepass_kernel(const uint32_t *__restrict__ src, const uint3
             continue;
         }
         const uint32_t at = base + (uint32_t)__popc(same & ((1u << lane) - 1u));
-        place[j] = at;
+        if (place) place[j] = at;
         row = max(row, at + 1u);
         float st = roundf(__fdiv_rn(dly[j], dt));
         if (st < 1.0f) st = 1.0f;
@@ -407,6 +407,7 @@ cudaError_t csr_scan(const uint32_t *counts, uint32_t n, uint32_t e, uint32_t *r
     return cudaGetLastError();
 }
 
+bool csr_list_short(uint64_t n_syn) { return n_syn <= (1ull << 29); }  // 10 GB of scratch
 bool csr_rows_short(uint32_t max_row) { return max_row <= kOrderMax; }
 
 cudaError_t csr_place_and_order(const DevSynapses &ds, const uint16_t *steps, const uint32_t *place,

@@ -31,12 +31,13 @@ struct CsrScalars {
 
 // Checks references, rounds delays to steps, counts synapses per source
 // (counts zeroed by the caller), gives each synapse a place of its own in its
-// source's row (place[n_syn], in no particular order) and finds the largest
+// source's row (place[n_syn], in no particular order; or null) and finds the largest
 // and smallest delay and the longest row.
 cudaError_t csr_prepass(const DevSynapses &ds, uint32_t *counts, uint32_t *place, uint16_t *steps, CsrScalars *sc,
                         cudaStream_t st);
-// Rows short enough for csr_place_and_order (16 bytes of scratch per
-// synapse); else csr_scatter.
+// Lists and rows short enough for csr_place_and_order (20 bytes of scratch per
+// synapse with the places); else csr_scatter, which needs none.
+bool csr_list_short(uint64_t n_syn);
 bool csr_rows_short(uint32_t max_row);
 cudaError_t csr_place_and_order(const DevSynapses &ds, const uint16_t *steps, const uint32_t *place,
                                 const uint32_t *rowptr, void *scratch, SynRec *syn_out, uint16_t *delay16_out,

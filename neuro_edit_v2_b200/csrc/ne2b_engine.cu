@@ -577,20 +577,22 @@ ne2b_status Engine::build_net(const ne2b_net_desc *net, const ne2b_config *cfg, 
         // the list's CSR sorted into place on the device (csrc/ne2b_csr.cu)
         NET_TRY(cuda_error(csr_scan(dc->counts, n, (uint32_t)h->e, (uint32_t *)d.rowptr, dc->cursor, dc->sums, bst),
                            "device CSR: row pointers"));
-        if (dc->short_rows) {
-            void *scratch = nullptr;
-            if (h->e) {
-                NET_TRY(cuda_error(cudaMallocAsync(&scratch, 16 * (size_t)h->e, bst), "cudaMallocAsync (device CSR)"));
-                const cudaError_t e = csr_place_and_order(dc->syn, dc->steps, dc->place, d.rowptr, scratch, (SynRec *)d.syn,
-                                                          (uint16_t *)d.delay16, int_ring_, wide, bst);
-                cudaFreeAsync(scratch, bst);
-                NET_TRY(cuda_error(e, "device CSR: place and order"));
-            }
-        } else
-        NET_TRY(cuda_error(csr_scatter(dc->syn, dc->steps, dc->cursor, (SynRec *)d.syn, (uint16_t *)d.delay16, int_ring_, wide,
-                                       dc->ticket, dc->done, dc->sc, 5000000000ull, bst),
-                           "device CSR: scatter"));
-        h->build_launches += (n ? 3 : 0) + (h->e ? (dc->short_rows ? 2 : 1) : 0);
+        void *scratch = nullptr;
+        if (dc->short_rows && h->e && cudaMallocAsync(&scratch, 16 * (size_t)h->e, bst) != cudaSuccess) {
+            cudaGetLastError();  // no room for the scratch: the scatter needs none
+            scratch = nullptr;
+        }
+        if (scratch) {
+            const cudaError_t e = csr_place_and_order(dc->syn, dc->steps, dc->place, d.rowptr, scratch, (SynRec *)d.syn,
+                                                      (uint16_t *)d.delay16, int_ring_, wide, bst);
+            cudaFreeAsync(scratch, bst);
+            NET_TRY(cuda_error(e, "device CSR: place and order"));
+        } else {
+            NET_TRY(cuda_error(csr_scatter(dc->syn, dc->steps, dc->cursor, (SynRec *)d.syn, (uint16_t *)d.delay16, int_ring_, wide,
+                                           dc->ticket, dc->done, dc->sc, 5000000000ull, bst),
+                               "device CSR: scatter"));
+        }
+        h->build_launches += (n ? 3 : 0) + (h->e ? (scratch ? 2 : 1) : 0);
     } else {
         NET_TRY(up((void *)d.rowptr, net->src_ptr, sizeof(uint32_t) * ((size_t)n + 1)));
     }

@@ -362,11 +362,12 @@ __global__ void augment_kernel(const float *__restrict__ x, const float *__restr
 // entry summed over the rows in order: a (F + 1 wide) and, from the last
 // column, the right-hand side.  4 x 4 entries per thread and cp.async as in
 // gram_kernel; the conversion to f64 is done once beforehand (on the way to
-// shared memory it took as long as the sums).  166 us at 1200 x 1080 with the
+// shared memory it took as long as the sums).  `more`: the sums go on from
+// those of earlier rows.  166 us at 1200 x 1080 with the
 // conversion, against 249 + 315 us with 2 x 2 entries per thread and a thread
 // per column for the bias and right-hand side.
 __global__ void __launch_bounds__(64) normal_kernel(const double *__restrict__ xa, uint32_t t, uint32_t f,
-                                                    uint32_t pitch, double *__restrict__ a,
+                                                    uint32_t pitch, bool more, double *__restrict__ a,
                                                     double *__restrict__ rhs) {
     __shared__ __align__(16) double si[2][kChunk][kTile], sj[2][kChunk][kTile];
     uint32_t bi, bj;
@@ -383,7 +384,18 @@ __global__ void __launch_bounds__(64) normal_kernel(const double *__restrict__ x
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    auto entry = [&](int p, int q) -> double * {  // where the sum of this thread's entry (p, q) is kept
+        const uint32_t i = i0 + spread4<kTile>(ty, p), j = j0 + spread4<kTile>(tx, q);
+        if (i > f || i > j || j > nf) return nullptr;
+        return j < nf ? a + (size_t)i * nf + j : rhs + i;
+    };
     double acc[4][4] = {};
+    if (more)  // the rows before these, summed by an earlier launch
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (const double *e = entry(p, q)) acc[p][q] = *e;
     stage(0u, 0u);
     for (uint32_t r0 = 0, buf = 0; r0 < t; r0 += kChunk, buf ^= 1u) {
         stage(r0 + kChunk, buf ^ 1u);
@@ -405,12 +417,8 @@ __global__ void __launch_bounds__(64) normal_kernel(const double *__restrict__ x
 #pragma unroll
     for (int p = 0; p < 4; ++p)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint32_t i = i0 + spread4<kTile>(ty, p), j = j0 + spread4<kTile>(tx, q);
-            if (i > f || i > j) continue;
-            if (j < nf) a[(size_t)i * nf + j] = acc[p][q];
-            else if (j == nf) rhs[i] = acc[p][q];
-        }
+        for (int q = 0; q < 4; ++q)
+            if (double *e = entry(p, q)) *e = acc[p][q];
 }
 
 // a[i][i] += add for every i; with `unbias`, a[f][f] then loses lambda again.
@@ -551,12 +559,17 @@ ne2b_status fit_binary_on_device(const float *x, uint32_t t, uint32_t f, const f
     NE2B_CUDA(cudaMemcpyAsync(y, y_host, sizeof(float) * t, cudaMemcpyHostToDevice, st));
     const uint32_t nt = (nf + 1u + kTile - 1u) / kTile;  // columns x, 1 and y
     const uint32_t pitch = (nf + 2u) / 2u * 2u;
+    // the f64 copy of at most 2 GB of rows at a time, summed on
+    const uint32_t rows = std::min(t, (uint32_t)std::max<uint64_t>(64u, (2ull << 30) / (8ull * pitch)));
     double *xa = nullptr;
-    NE2B_TRY(buf.get(&xa, (size_t)t * pitch));
-    for (uint32_t r0 = 0; r0 < t; r0 += 65535u)  // rows along grid y
-        augment_kernel<<<dim3(std::min(64u, (pitch + 255u) / 256u), std::min(65535u, t - r0)), 256, 0, st>>>(
-            x + (size_t)r0 * f, y + r0, t - r0, f, pitch, xa + (size_t)r0 * pitch);
-    normal_kernel<<<nt * (nt + 1) / 2, 64, 0, st>>>(xa, t, f, pitch, a, b);
+    NE2B_TRY(buf.get(&xa, (size_t)rows * pitch));
+    for (uint32_t r0 = 0; r0 < t; r0 += rows) {
+        const uint32_t nr = std::min(rows, t - r0);
+        for (uint32_t g0 = 0; g0 < nr; g0 += 65535u)  // rows along grid y
+            augment_kernel<<<dim3(std::min(64u, (pitch + 255u) / 256u), std::min(65535u, nr - g0)), 256, 0, st>>>(
+                x + (size_t)(r0 + g0) * f, y + r0 + g0, nr - g0, f, pitch, xa + (size_t)g0 * pitch);
+        normal_kernel<<<nt * (nt + 1) / 2, 64, 0, st>>>(xa, nr, f, pitch, r0 > 0u, a, b);
+    }
     const double lam = (double)lambda;
     diag_kernel<<<(nf + 255) / 256, 256, 0, st>>>(a, nf, lam, true, lam);
     NE2B_CUDA(cudaMemcpyAsync(a0, a, sizeof(double) * nf * nf, cudaMemcpyDeviceToDevice, st));

@@ -168,12 +168,16 @@ ne2b_status ne2b_external(ne2b_sim *sim, float *out);
 ne2b_status ne2b_set_noise(ne2b_sim *sim, float rate_hz, float kick_mv);
 ne2b_status ne2b_set_gauss_noise(ne2b_sim *sim, float sd);                 /* new */
 
-/* Step kernel selection (new): NE2B_KERNEL_AUTO runs the streaming kernel
- * (one launch per step), which ne2b_autotune may replace by the resident
- * persistent kernel where that measures faster; the other two force one
- * (RESIDENT fails with NE2B_UNSUPPORTED when the nets' state does not fit
- * in shared memory).  *resident reports which kernel runs.  The environment variable NE2B_KERNEL=stream|resident sets
- * the initial mode of every handle. */
+/* Step kernel selection (new): NE2B_KERNEL_AUTO, with no tile shape set,
+ * picks by size: nets of up to 16 x 1024 neurons (16 x 4096 each in a batch
+ * or server) run many steps per launch on thread-block clusters, larger
+ * single nets a streaming kernel (one launch per step) with or without
+ * deferred delivery; ne2b_autotune may replace the choice where another
+ * kernel measures faster.  STREAM forces the streaming kernel, RESIDENT the
+ * cooperative resident kernel (NE2B_UNSUPPORTED when the nets' state does
+ * not fit in shared memory; *resident reports whether it runs).  Results are
+ * the same (bit for bit with the int32 ring).  The environment variable
+ * NE2B_KERNEL=stream|resident sets the initial mode of every handle. */
 enum { NE2B_KERNEL_AUTO = 0, NE2B_KERNEL_STREAM = 1, NE2B_KERNEL_RESIDENT = 2 };
 ne2b_status ne2b_set_kernel_mode(ne2b_sim *sim, int32_t mode);
 ne2b_status ne2b_kernel_mode(ne2b_sim *sim, int32_t *mode, int32_t *resident);

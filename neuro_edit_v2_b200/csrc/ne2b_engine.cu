@@ -384,7 +384,7 @@ void Engine::discard_net(NetHost *h, cudaStream_t st) {
 ne2b_status Engine::attach_net(NetHost *h, uint32_t *slot_out, bool rebuild) {
     if (!fixed_grid) {  // pinned with the net, not by the first read of its state (the server's results go another way)
         std::lock_guard<std::mutex> lk(fetch_mu_);
-        NE2B_TRY(fetch_reserve(64 + std::min(kFetchPinned, sizeof(float) * (size_t)h->n)));
+        (void)fetch_reserve(64 + std::min(kFetchPinned, sizeof(float) * (size_t)h->n));  // reads go without it if need be
     }
     uint32_t slot = nets_cap_;
     for (uint32_t j = 0; j < nets_cap_; ++j)
@@ -1091,7 +1091,10 @@ ne2b_status Engine::plan_defer() {
         h->urgent = 0;
         if (d.hop == 1u) {
             const size_t words = h->n_pad / 32 + 1;  // the last one counts
-            NE2B_CUDA(cudaMallocAsync(&p, sizeof(uint32_t) * words, stream_));
+            if (cudaMallocAsync(&p, sizeof(uint32_t) * words, stream_) != cudaSuccess) {
+                cudaGetLastError();  // no room: the fused kernel needs none
+                return NE2B_OK;
+            }
             h->allocs.push_back(p);
             uint32_t *bits = (uint32_t *)p, count = 0;
             NE2B_CUDA(cudaMemsetAsync(bits, 0, sizeof(uint32_t) * words, stream_));
@@ -1103,10 +1106,13 @@ ne2b_status Engine::plan_defer() {
             d.urgent = bits;
         }
         if (h->urgent * 4 <= (int64_t)h->n) {
-            NE2B_CUDA(cudaMallocAsync(&p, sizeof(uint2_pod) * 3 * (size_t)h->n_pad + 16, stream_));
-            h->allocs.push_back(p);
-            d.slist = (uint2_pod *)p;
-            d.scount = (uint32_t *)(d.slist + 3 * (size_t)h->n_pad);
+            if (cudaMallocAsync(&p, sizeof(uint2_pod) * 3 * (size_t)h->n_pad + 16, stream_) == cudaSuccess) {
+                h->allocs.push_back(p);
+                d.slist = (uint2_pod *)p;
+                d.scount = (uint32_t *)(d.slist + 3 * (size_t)h->n_pad);
+            } else {
+                cudaGetLastError();
+            }
         }
         NE2B_TRY(upload_net(*h));
     }
@@ -1240,7 +1246,12 @@ ne2b_status Engine::fetch_reserve(size_t bytes) {
     if (fetch_pin_) cudaFreeHost(fetch_pin_);
     fetch_pin_ = nullptr;
     fetch_cap_ = 0;
-    NE2B_CUDA(cudaMallocHost(&fetch_pin_, cap));
+    const cudaError_t e = cudaMallocHost(&fetch_pin_, cap);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        fetch_pin_ = nullptr;
+        return cuda_error(e, "pinned read buffer");
+    }
     fetch_cap_ = cap;
     return NE2B_OK;
 }
@@ -1254,8 +1265,7 @@ ne2b_status Engine::fetch_reserve(size_t bytes) {
 ne2b_status Engine::fetch(void *out, const void *dev, size_t bytes, bool check) {
     constexpr size_t kFlag = 64;  // the flag's place, before the data
     std::unique_lock<std::mutex> lk(fetch_mu_, std::try_to_lock);
-    if (lk.owns_lock() && bytes <= kFetchPinned) {
-        NE2B_TRY(fetch_reserve(kFlag + bytes));
+    if (lk.owns_lock() && bytes <= kFetchPinned && fetch_reserve(kFlag + bytes) == NE2B_OK) {
         uint8_t *pin = (uint8_t *)fetch_pin_;
         if (bytes) NE2B_CUDA(cudaMemcpyAsync(pin + kFlag, dev, bytes, cudaMemcpyDeviceToHost, stream_));
         if (check) NE2B_CUDA(cudaMemcpyAsync(pin, d_err_, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream_));

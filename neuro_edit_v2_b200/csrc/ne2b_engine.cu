@@ -862,7 +862,7 @@ int Engine::step_variant(const TileShape &s) const {
 // tk, pidx: 4 B per neuron) in dynamic shared memory.  Chooses the most
 // blocks per SM whose shared memory still fits; false when nothing fits.
 bool Engine::plan_resident(std::vector<Tile> &tiles, std::vector<uint32_t> &block_tiles) {
-    // AUTO streams: on B200 the resident kernel's software grid barrier
+    // AUTO never picks it: on B200 the resident kernel's software grid barrier
     // (an arrival atomic and an acquire poll, two L2 round trips) costs more
     // than a kernel boundary in a graph with programmatic dependent launch
     // (10k neurons: 2.9 against 1.4 us per step; 100k: 3.1 against 1.9).

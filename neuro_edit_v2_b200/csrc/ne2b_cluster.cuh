@@ -13,11 +13,22 @@
 // B steps (a hop): a spike of step t lands in slot t + d, d >= B, so every
 // slot of steps [T, T + B) is complete when step T starts.  Each neuron then
 // runs B steps at once from registers, its ring words loaded ahead, and the
-// spikes of the B steps are listed in shared memory and delivered together.
-// A second barrier separates the hop's ring reads from its deliveries,
-// because a delay close to the ring depth lands in a slot that another block
-// of the cluster may not have read yet.  With B = 1 (ONE) that cannot happen
-// (d < D), so each warp delivers its own spikes at once.
+// spikes of the B steps are listed in shared memory and delivered together
+// after a block barrier.  With B = 1 (ONE) each warp delivers its own spikes
+// at once.  The nets that run here have kRingSpare ring slots beyond their
+// longest delay, so no delivery of a hop lands in a slot that the hop reads.
+//
+// What orders the ring between blocks (ne2b_layout.h, release_due):
+//   add -> read   an add of hop h is read in a later hop: the warp that added
+//                 releases at the barrier between them;
+//   read, clear -> add   a slot read and cleared at step t is added to again
+//                 at step t + kRingSpare + 1 at the earliest: every warp
+//                 releases often enough that one of its releases lies between.
+// Every warp acquires at every barrier.  The spike lists of a block are
+// written before, and read after, a block barrier; they are written again
+// after the cluster barrier, at which the warps that read them (they deliver)
+// release.  The hop's counters take turns among three sets: a set is cleared
+// one block barrier after its last read and one before its next use.
 //
 // The arithmetic per neuron is process_tile's, in its order (ne2b_step.cuh).
 #pragma once
@@ -40,15 +51,15 @@ __device__ __forceinline__ uint32_t cluster_blocks() {
     return r;
 }
 // All threads of the cluster (of the block when it is alone).  Every warp
-// acquires; only a warp that wrote to the ring releases, because the release
-// waits for its writes to land: 0.16 us for 16 blocks of 512 threads without
-// it, 0.6 us with ring writes in flight.
-__device__ __forceinline__ void cluster_barrier(uint32_t blocks, bool wrote) {
+// acquires; a relaxed arrival orders nothing that the warp did before it.
+// 0.16 us for 16 blocks of 512 threads when no warp releases, 0.3 when all do,
+// 0.6 with ring writes in flight.
+__device__ __forceinline__ void cluster_barrier(uint32_t blocks, bool release) {
     if (blocks == 1u) {
         __syncthreads();
         return;
     }
-    if (wrote) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (release) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     else asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -119,15 +130,15 @@ __global__ void __launch_bounds__(kClMaxThreads) cluster_kernel(const EngineDev 
     const uint32_t n = nd.n, n_pad = nd.n_pad, D = nd.D, m = cn.m, B = ONE ? 1u : nd.hop;
     const uint32_t start = min(rank * m, n_pad), cnt = min(m, n_pad - start);  // multiples of 32
 
-    // the hop's spikes: [step] counters, then [step][m] local neurons (u16);
-    // then (LOOP) the state
-    uint32_t *scnt = reinterpret_cast<uint32_t *>(smem);
-    uint16_t *slist = reinterpret_cast<uint16_t *>(scnt + (ONE ? 0u : kMaxHop));
+    // the hop's spikes: three sets of [step] counters, then [step][m] local
+    // neurons (u16); then (LOOP) the state
+    uint32_t *sets = reinterpret_cast<uint32_t *>(smem);
+    uint16_t *slist = reinterpret_cast<uint16_t *>(sets + (ONE ? 0u : 3u * kMaxHop));
     float *sv = reinterpret_cast<float *>(slist + (ONE ? 0u : m * B));
     float *su = sv + m, *ss = su + m;
     uint16_t *slast = reinterpret_cast<uint16_t *>(ss + m), *spi = slast + m;
     if (!ONE) {
-        if (threadIdx.x < kMaxHop) scnt[threadIdx.x] = 0u;
+        for (uint32_t w = threadIdx.x; w < 3u * kMaxHop; w += T) sets[w] = 0u;
         __syncthreads();
     }
 
@@ -205,9 +216,11 @@ __global__ void __launch_bounds__(kClMaxThreads) cluster_kernel(const EngineDev 
         glanes = e_avg <= 32u ? 8u : e_avg <= 64u ? 16u : 32u;
     }
 
+    uint32_t set = 0u, since = 0u;  // this hop's counters; steps since every warp released
     for (uint32_t s0 = 0; s0 < steps;) {
         const uint32_t nb = ONE ? 1u : min(min(B, steps - s0), wleft);  // a window ends with a hop
-        bool wrote = false, zeroed = false;  // ring words written by this warp / thread
+        uint32_t *scnt = sets + set * kMaxHop;
+        bool wrote = false;  // this warp added to the ring
         for (uint32_t o0 = 0; o0 < (LOOP ? cnt : 1u); o0 += T) {
             const uint32_t o = o0 + threadIdx.x, i = start + o;
             if (LOOP) {
@@ -234,10 +247,7 @@ __global__ void __launch_bounds__(kClMaxThreads) cluster_kernel(const EngineDev 
             for (uint32_t b = 0; b < nb; ++b) {
                 const float arr = INT ? __fmul_rn(__int2float_rn((int)w0), 0x1p-12f)  // rt_get, kernels.rs:60
                                       : __uint_as_float(w0);
-                if (w0 != 0u) {
-                    ringw[(size_t)slot * n_pad + i] = 0u;
-                    zeroed = true;
-                }
+                if (w0 != 0u) ringw[(size_t)slot * n_pad + i] = 0u;
                 w0 = w1;
                 w1 = fetch(b + 2u);
                 const float sc = __fadd_rn(s, arr);
@@ -330,12 +340,11 @@ __global__ void __launch_bounds__(kClMaxThreads) cluster_kernel(const EngineDev 
             wleft = nd.win_steps;
             ++widx;
         }
-        wrote = __any_sync(0xffffffffu, zeroed) || wrote;
         if (!ONE) {
-            // every block has read its slots of the hop before any delivery
-            // of it: a delay above D - nb lands in one of them
-            cluster_barrier(C, wrote);
-            wrote = false;
+            __syncthreads();  // the block's lists are complete
+            const uint32_t after = set == 0u ? 2u : set - 1u;  // the set of the hop after next
+            if (threadIdx.x < kMaxHop) sets[after * kMaxHop + threadIdx.x] = 0u;
+            set = set == 2u ? 0u : set + 1u;
             // the block's spikes of the hop, one per group of lanes
             uint32_t total = 0;
             for (uint32_t b = 0; b < nb; ++b) total += scnt[b];
@@ -349,12 +358,11 @@ __global__ void __launch_bounds__(kClMaxThreads) cluster_kernel(const EngineDev 
                 wrote = true;
             }
             wrote = __any_sync(0xffffffffu, wrote);
-            if (total) {  // uniform: the counters are cleared once all have read them
-                __syncthreads();
-                if (threadIdx.x < kMaxHop) scnt[threadIdx.x] = 0u;
-            }
         }
-        cluster_barrier(C, wrote);  // the deliveries have landed before the next hop reads
+        since += nb;
+        const bool due = release_due(since, B);
+        cluster_barrier(C, wrote || due);  // the deliveries have landed before the next hop reads
+        if (due) since = 0u;
         tm = add_mod(tm, nb, D);
         s0 += nb;
     }

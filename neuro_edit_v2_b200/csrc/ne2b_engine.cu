@@ -534,7 +534,19 @@ ne2b_status Engine::build_net(const ne2b_net_desc *net, const ne2b_config *cfg, 
     NET_TRY(alloc(&p, sizeof(float) * np)); d.u0 = (const float *)p;
     NET_TRY(alloc(&p, sizeof(uint16_t) * np)); d.pidx = (const uint16_t *)p;
     NET_TRY(alloc(&p, sizeof(unsigned long long) * np)); d.pn_total = (unsigned long long *)p;
-    NET_TRY(alloc(&p, sizeof(uint32_t) * (size_t)h->D * np)); d.ring = p;
+    h->slots = h->D;
+    if (!any_tau && np <= 16u * kClMaxNeurons) {  // (a net without the spare slots keeps to the other kernels)
+        const size_t bytes = sizeof(uint32_t) * (size_t)(h->D + kRingSpare) * np;
+        if (np && cudaMallocAsync(&d.ring, bytes, bst) == cudaSuccess) {
+            h->allocs.push_back(d.ring);
+            h->dev_bytes += bytes;
+            h->slots = h->D + kRingSpare;
+        } else {
+            cudaGetLastError();
+            d.ring = nullptr;
+        }
+    }
+    if (!d.ring) { NET_TRY(alloc(&p, sizeof(uint32_t) * (size_t)h->D * np)); d.ring = p; }
     NET_TRY(alloc(&p, sizeof(uint32_t) * ((size_t)n + 1))); d.rowptr = (const uint32_t *)p;
     NET_TRY(alloc(&p, sizeof(SynRec) * h->e)); d.syn = (const SynRec *)p;
     // delays past 8 bits, or targets past 24, do not fit the packed record
@@ -679,7 +691,7 @@ ne2b_status Engine::build_net(const ne2b_net_desc *net, const ne2b_config *cfg, 
         NET_TRY(alloc(&p, sizeof(float) * nx)); d.xw = (const float *)p;
         NET_TRY(up(p, xw.data(), sizeof(float) * nx));
         NET_TRY(alloc(&p, sizeof(float) * nx)); d.xsyn = (float *)p;
-        NET_TRY(alloc(&p, sizeof(uint32_t) * (size_t)h->D * d.xwords)); d.xpend = (uint32_t *)p;
+        NET_TRY(alloc(&p, sizeof(uint32_t) * (size_t)h->slots * d.xwords)); d.xpend = (uint32_t *)p;
     }
     tp[4] = now_ms();
     // stimulus routing
@@ -720,12 +732,12 @@ ne2b_status Engine::build_net(const ne2b_net_desc *net, const ne2b_config *cfg, 
     }
     d.n = n;
     d.n_pad = np;
-    d.D = h->D;
+    d.D = h->slots;
     d.t_end = h->t_end;
     d.seed = cfg->seed;
     d.n_inputs = net->n_inputs;
     d.rec_rows = rec_rows;
-    d.hop = std::max(1u, std::min(std::min(mind, kMaxHop), h->D - 1));  // every slot of a hop is its own
+    d.hop = std::max(1u, std::min(std::min(mind, kMaxHop), h->D - 1));
     set_step(d, 0);
     d.dt = cfg->dt_ms;
     d.decay_s = host_decay(cfg->dt_ms, cfg->synapse_tau_ms);
@@ -765,7 +777,7 @@ ne2b_status Engine::build_net(const ne2b_net_desc *net, const ne2b_config *cfg, 
     // initial state (cpu.rs:158-183), on the build stream
     NET_TRY(cuda_error(launch_reset_neurons(d, bst), "reset kernel"));
     h->build_launches += np ? 1 : 0;
-    NET_TRY(cuda_error(cudaMemsetAsync(d.ring, 0, sizeof(uint32_t) * (size_t)h->D * np, bst), "memset ring"));
+    NET_TRY(cuda_error(cudaMemsetAsync(d.ring, 0, sizeof(uint32_t) * (size_t)h->slots * np, bst), "memset ring"));
     if (d.rec_bits)
         NET_TRY(cuda_error(cudaMemsetAsync(d.rec_bits, 0, sizeof(uint32_t) * (size_t)rec_rows * (np / 32), bst),
                            "memset record"));
@@ -774,7 +786,7 @@ ne2b_status Engine::build_net(const ne2b_net_desc *net, const ne2b_config *cfg, 
                            "memset windows"));
     if (h->nx) {
         NET_TRY(cuda_error(cudaMemsetAsync(d.xsyn, 0, sizeof(float) * h->nx, bst), "memset xsyn"));
-        NET_TRY(cuda_error(cudaMemsetAsync(d.xpend, 0, sizeof(uint32_t) * (size_t)h->D * d.xwords, bst),
+        NET_TRY(cuda_error(cudaMemsetAsync(d.xpend, 0, sizeof(uint32_t) * (size_t)h->slots * d.xwords, bst),
                            "memset xsyn arrivals"));
     }
     NET_TRY(sg.close());
@@ -997,7 +1009,7 @@ bool Engine::plan_cluster(std::vector<ClusterNet> &plan) {
     uint32_t largest = 0;
     for (const NetHost *h : nets_)
         if (h) {
-            if (h->nx) return false;
+            if (h->nx || (h->n_pad && h->slots < h->D + kRingSpare)) return false;
             total += h->n_pad;
             largest = std::max(largest, h->n_pad);
         }
@@ -1218,13 +1230,13 @@ ne2b_status Engine::reset_net(uint32_t slot) {
     NetDev &d = h.dev;
     NE2B_CUDA(launch_reset_neurons(d, stream_));
     launches_ += d.n_pad ? 1 : 0;
-    NE2B_CUDA(cudaMemsetAsync(d.ring, 0, sizeof(uint32_t) * (size_t)h.D * h.n_pad, stream_));
+    NE2B_CUDA(cudaMemsetAsync(d.ring, 0, sizeof(uint32_t) * (size_t)h.slots * h.n_pad, stream_));
     if (d.rec_bits) NE2B_CUDA(cudaMemsetAsync(d.rec_bits, 0, sizeof(uint32_t) * (size_t)d.rec_rows * (h.n_pad / 32), stream_));
     if (d.win_out) NE2B_CUDA(cudaMemsetAsync(d.win_out, 0, sizeof(uint16_t) * (size_t)d.max_windows * h.n_pad, stream_));
     if (d.trace_f) NE2B_CUDA(cudaMemsetAsync(d.trace_f, 0, sizeof(float) * h.n_pad, stream_));
     if (h.nx) {
         NE2B_CUDA(cudaMemsetAsync(d.xsyn, 0, sizeof(float) * h.nx, stream_));
-        NE2B_CUDA(cudaMemsetAsync(d.xpend, 0, sizeof(uint32_t) * (size_t)h.D * d.xwords, stream_));
+        NE2B_CUDA(cudaMemsetAsync(d.xpend, 0, sizeof(uint32_t) * (size_t)h.slots * d.xwords, stream_));
     }
     // cpu.rs:176-183: the watch history and the grid marks start over
     h.watch_t0 = 0;
@@ -1759,14 +1771,14 @@ ne2b_status Engine::snapshot(EngineSnapshot &snap) {
         NE2B_TRY(grab(d.tk, 2 * np));
         NE2B_TRY(grab(d.trace_f, d.trace_f ? 4 * np : 0));
         NE2B_TRY(grab(d.pn_total, 8 * np));
-        NE2B_TRY(grab(d.ring, 4 * (size_t)h->D * np));
+        NE2B_TRY(grab(d.ring, 4 * (size_t)h->slots * np));
         NE2B_TRY(grab(d.rec_bits, d.rec_bits ? 4 * (size_t)d.rec_rows * (np / 32) : 0));
         NE2B_TRY(grab(d.wcount, d.wcount ? 4 * np : 0));
         NE2B_TRY(grab(d.win_out, d.win_out ? 2 * (size_t)d.max_windows * np : 0));
         NE2B_TRY(grab(d.xsyn, 4 * (size_t)h->nx));
         NE2B_TRY(grab(d.watch_ring, d.watch_ring ? 8 * (size_t)d.watch_n * kWatchCap : 0));
         NE2B_TRY(grab(d.gw_ls, d.gw_ls ? 4 * (size_t)std::max<uint32_t>(h->gw_ptr.back(), 1) : 0));
-        NE2B_TRY(grab(d.xpend, 4 * (size_t)h->D * d.xwords));
+        NE2B_TRY(grab(d.xpend, 4 * (size_t)h->slots * d.xwords));
         snap.hosts.push_back({h->slot, h->t, h->dev});
     }
     return NE2B_OK;

@@ -57,6 +57,7 @@ struct NetHost {
     NetDev dev{};             // host mirror of the device descriptor
     uint32_t slot = 0;        // index in the engine's net array
     uint32_t n = 0, n_pad = 0, D = 0, n_inputs = 0;
+    uint32_t slots = 0;       // ring slots on the device: D, or D + kRingSpare where the cluster kernel may run
     uint64_t e = 0;
     int64_t urgent = -1;      // neurons with a synapse of delay 1, -1 before they are counted
     uint32_t nx = 0;          // synapses with their own tau (XSyn)

@@ -133,7 +133,7 @@ struct alignas(16) NetDev {
     long long stim_t0;          // step of stim_buf row 0
     unsigned long long seed;
     unsigned long long noise_step;  // step part of the noise base at t (set_step)
-    uint32_t n, n_pad, D, tmod;  // tmod = t % D
+    uint32_t n, n_pad, D, tmod;  // D: ring slots, past the longest delay; tmod = t % D
     uint32_t n_inputs, stim_len;
     uint32_t rec_rows, win_steps, max_windows, flags;
     float dt, pkick, kick, decay_s, decay_t, gauss_k;
@@ -147,6 +147,11 @@ struct alignas(16) NetDev {
     uint32_t hop;  // steps the cluster kernel runs between barriers: the shortest delay, at most kMaxHop
 };
 constexpr uint32_t kMaxHop = 16;
+// Ring slots beyond the longest delay + 1 of a net that may run on the cluster
+// kernel: slot t is read and cleared at step t and next added to at step
+// t + kRingSpare + 1 or later.
+constexpr uint32_t kRingSpare = 15;
+static_assert(kMaxHop <= kRingSpare + 1u, "no delivery of a hop lands in a slot that the hop reads");
 constexpr uint32_t kClMaxNeurons = 4096;  // neurons of a cluster kernel block, at most
 constexpr uint32_t kClMinNeurons = 256;   // below this a net is not split over more blocks
 
@@ -159,6 +164,13 @@ constexpr uint32_t kClMinNeurons = 256;   // below this a net is not split over 
 // (sim/src/state.rs:285-288).
 constexpr unsigned long long kNoiseStepMul = 0xBF58476D1CE4E5B9ull;
 constexpr unsigned long long kNoiseSeedMul = 0x94D049BB133111EBull;
+
+// Whether every warp of a cluster releases at the barrier that ends a hop,
+// `since` steps after the last barrier where every warp did (or the launch's
+// start), when the coming hops have at most `hop` steps.  Reads at or after
+// that barrier's step r may meet adds from step r + kRingSpare + 1 on; without
+// a release here the next hop still ends before that step.
+NE2B_HD constexpr bool release_due(uint32_t since, uint32_t hop) { return since + hop > kRingSpare + 1u; }
 
 // Sets t and every phase derived from it (tmod, rphase, wphase, widx0, and
 // the noise base's step part t * kNoiseStepMul + seed * kNoiseSeedMul, from

@@ -56,10 +56,10 @@ struct ClusterShape {
     uint32_t threads;
     bool loop, one;
 };
-// Its shared memory: the hop's spike counters and lists (u16 per neuron and
+// Its shared memory: three sets of spike counters, the lists (u16 per neuron and
 // step), then (loop) the state (16 bytes per neuron).
 inline uint32_t cluster_smem(uint32_t m, uint32_t hop, const ClusterShape &s) {
-    return (s.one ? 0u : kMaxHop * 4u + m * hop * 2u) + (s.loop ? m * 16u : 0u);
+    return (s.one ? 0u : 3u * kMaxHop * 4u + m * hop * 2u) + (s.loop ? m * 16u : 0u);
 }
 
 template <bool INT, bool ADEX>

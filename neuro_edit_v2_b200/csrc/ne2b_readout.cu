@@ -212,13 +212,15 @@ __global__ void __launch_bounds__(64) gram_kernel(const double *__restrict__ xc,
 // move up one place per j) so that a launch's code, which runs once, is
 // short.  The factored diagonal block goes to dblk, because other blocks may
 // still be reading the original; the trailing update puts it in place (the
-// last panel, one block, does so itself).  A non-positive pivot raises *bad
-// (the matrix is not positive definite).
+// last panel, one block, does so itself).  A non-positive pivot (the matrix is
+// not positive definite) raises bad[1], which only the update tests; the
+// update passes it on to bad[0], which only the next panel tests.  So no
+// launch tests a flag that it may be setting, and all threads find the same.
 constexpr uint32_t kPanelCols = 96;  // columns right of the panel per block
 __global__ void __launch_bounds__(32 + kPanelCols) chol_panel_kernel(double *g, uint32_t n, uint32_t p,
                                                                      double *__restrict__ dblk, unsigned int *bad) {
     __shared__ double sd[kPanel][2u * kPanel];  // sd[j][k] = U[p + j][p + k], k >= j; read up to k = j + 31
-    if (*bad) return;  // set by an earlier panel: uniform
+    if (bad[0]) return;  // an earlier panel failed
     const uint32_t nb = min(kPanel, n - p), lane = threadIdx.x & 31u;
     const bool diag = threadIdx.x < 32u;
     // columns to the right exist only past a full panel
@@ -258,16 +260,19 @@ __global__ void __launch_bounds__(32 + kPanelCols) chol_panel_kernel(double *g, 
         }
         __syncthreads();
     }
-    if (stop && blockIdx.x == 0u && lane == 0u) atomicExch(bad, 1u);
+    if (diag && stop && blockIdx.x == 0u && lane == 0u) bad[1] = 1u;
 }
 
 // The trailing upper triangle past a full panel: G[k][i] -= U[p + j][k]
 // U[p + j][i] for j = 0..31 in order, from registers (one read and one write
 // of the matrix per 32 rows).
 __global__ void __launch_bounds__(256) chol_update_kernel(double *g, uint32_t n, uint32_t p,
-                                                          const double *__restrict__ dblk, const unsigned int *bad) {
+                                                          const double *__restrict__ dblk, unsigned int *bad) {
     __shared__ __align__(16) double sk[kPanel][kUpdTile], si[kPanel][kUpdTile];
-    if (*bad) return;
+    if (bad[1]) {
+        if (blockIdx.x == 0u && threadIdx.x == 0u) bad[0] = 1u;
+        return;
+    }
     if (blockIdx.x == 0u)  // the panel's diagonal block, which nothing here reads
         for (uint32_t e = threadIdx.x; e < kPanel * kPanel; e += 256u)
             if (e % kPanel >= e / kPanel) g[(size_t)(p + e / kPanel) * n + p + e % kPanel] = dblk[e];
@@ -524,9 +529,9 @@ void keep_workspace(int device) {
 }
 
 // G = U^T U in place of the upper triangle; true when G is positive definite.
-// dblk: scratch, 32 x 32.
+// dblk: scratch, 32 x 32; bad: two flags.
 ne2b_status cholesky(double *g, uint32_t n, double *dblk, unsigned int *bad, cudaStream_t st, bool *pd) {
-    NE2B_CUDA(cudaMemsetAsync(bad, 0, sizeof(unsigned int), st));
+    NE2B_CUDA(cudaMemsetAsync(bad, 0, 2 * sizeof(unsigned int), st));
     for (uint32_t p = 0; p < n; p += kPanel) {
         const uint32_t right = n - std::min(n, p + kPanel);  // columns right of the panel
         chol_panel_kernel<<<std::max(1u, (right + kPanelCols - 1u) / kPanelCols), 32 + kPanelCols, 0, st>>>(g, n, p, dblk, bad);
@@ -535,7 +540,7 @@ ne2b_status cholesky(double *g, uint32_t n, double *dblk, unsigned int *bad, cud
     }
     NE2B_CUDA(cudaGetLastError());
     unsigned int bad_h = 0;
-    NE2B_CUDA(cudaMemcpyAsync(&bad_h, bad, sizeof bad_h, cudaMemcpyDeviceToHost, st));
+    NE2B_CUDA(cudaMemcpyAsync(&bad_h, bad + 1, sizeof bad_h, cudaMemcpyDeviceToHost, st));
     NE2B_CUDA(cudaStreamSynchronize(st));
     *pd = bad_h == 0;
     return NE2B_OK;
@@ -553,7 +558,7 @@ ne2b_status fit_binary_on_device(const float *x, uint32_t t, uint32_t f, const f
     NE2B_TRY(buf.get(&a0, (size_t)nf * nf));
     NE2B_TRY(buf.get(&b, nf));
     NE2B_TRY(buf.get(&y, t));
-    NE2B_TRY(buf.get(&bad, 1));
+    NE2B_TRY(buf.get(&bad, 2));
     double *dblk = nullptr;
     NE2B_TRY(buf.get(&dblk, (size_t)kPanel * kPanel));
     NE2B_CUDA(cudaMemcpyAsync(y, y_host, sizeof(float) * t, cudaMemcpyHostToDevice, st));
@@ -615,7 +620,7 @@ ne2b_status fit_on_device(const float *x, uint32_t t, uint32_t f, const uint32_t
     NE2B_TRY(buf.get(&g, (size_t)t * t));
     NE2B_TRY(buf.get(&a, (size_t)t * k));
     NE2B_TRY(buf.get(&w, (size_t)f * k));
-    NE2B_TRY(buf.get(&bad, 1));
+    NE2B_TRY(buf.get(&bad, 2));
     double *dblk = nullptr;
     NE2B_TRY(buf.get(&dblk, (size_t)kPanel * kPanel));
     col_mean_kernel<<<(f + 31) / 32, 128, 0, st>>>(x, t, f, mu);

@@ -35,13 +35,12 @@
 #include <string.h>
 
 #include <algorithm>
-#include <mutex>
-#include <type_traits>
 #include <vector>
 
 #include "ne2b_engine.h"
 #include "ne2b_handles.h"
 #include "ne2b_solve.h"
+#include "ne2b_workspace.h"
 
 #define NE2B_CUDA(call)                                      \
     do {                                                     \
@@ -465,57 +464,6 @@ struct DevBuf {
     }
 };
 
-// Pinned host memory for a fit's factor, so that its copy runs at the link's
-// rate and the host neither zeroes nor faults in fresh pages.  One buffer of
-// at most kPinnedKeep stays for the next fit of the process; a fit that finds
-// it taken (another thread's) or needs more allocates its own and frees it.
-class PinnedScratch {
-  public:
-    ~PinnedScratch() {
-        if (!p_) return;
-        {
-            std::lock_guard<std::mutex> lk(mu());
-            if (cap_ <= kPinnedKeep && cap_ >= kept().cap) {
-                std::swap(p_, kept().p);
-                std::swap(cap_, kept().cap);
-            }
-        }
-        if (p_) cudaFreeHost(p_);
-    }
-    ne2b_status get(size_t bytes, double **out) {
-        {
-            std::lock_guard<std::mutex> lk(mu());
-            if (kept().cap >= bytes) {
-                std::swap(p_, kept().p);
-                std::swap(cap_, kept().cap);
-            }
-        }
-        if (!p_) {
-            NE2B_CUDA(cudaHostAlloc(&p_, bytes, cudaHostAllocPortable));
-            cap_ = bytes;
-        }
-        *out = (double *)p_;
-        return NE2B_OK;
-    }
-
-  private:
-    static constexpr size_t kPinnedKeep = (size_t)64 << 20;
-    struct Kept {
-        void *p = nullptr;
-        size_t cap = 0;
-    };
-    static std::mutex &mu() {
-        static std::mutex m;
-        return m;
-    }
-    static Kept &kept() {
-        static Kept k;
-        return k;
-    }
-    void *p_ = nullptr;
-    size_t cap_ = 0;
-};
-
 // The default pool keeps up to this much freed memory for the next call
 // (unless it already keeps more): without it each fit maps its workspaces
 // anew.
@@ -589,9 +537,9 @@ ne2b_status fit_binary_on_device(const float *x, uint32_t t, uint32_t f, const f
         for (uint32_t i = 0; i < nf; ++i) w_out[i] = 0.0;
         return NE2B_OK;
     }
-    PinnedScratch pin;
-    double *u = nullptr;
-    NE2B_TRY(pin.get(sizeof(double) * ((size_t)nf * nf + nf), &u));
+    HostWorkspace host;
+    double *u = (double *)host.get(sizeof(double) * ((size_t)nf * nf + nf));
+    if (!u) return set_error(NE2B_ENOMEM, "host allocation failed");
     double *bh = u + (size_t)nf * nf;
     NE2B_CUDA(cudaMemcpyAsync(u, a, sizeof(double) * nf * nf, cudaMemcpyDeviceToHost, st));
     NE2B_CUDA(cudaMemcpyAsync(bh, b, sizeof(double) * nf, cudaMemcpyDeviceToHost, st));
@@ -636,9 +584,9 @@ ne2b_status fit_on_device(const float *x, uint32_t t, uint32_t f, const uint32_t
     NE2B_CUDA(cudaMemcpyAsync(mu_h.data(), mu, sizeof(double) * f, cudaMemcpyDeviceToHost, st));
     for (uint32_t r = 0; r < t; ++r) ybar[labels[r]] += 1.0 / (double)t;
     if (pd) {
-        PinnedScratch pin;
-        double *u = nullptr;
-        NE2B_TRY(pin.get(sizeof(double) * (size_t)t * t, &u));
+        HostWorkspace host;
+        double *u = (double *)host.get(sizeof(double) * (size_t)t * t);
+        if (!u) return set_error(NE2B_ENOMEM, "host allocation failed");
         NE2B_CUDA(cudaMemcpyAsync(u, g, sizeof(double) * (size_t)t * t, cudaMemcpyDeviceToHost, st));
         NE2B_CUDA(cudaStreamSynchronize(st));
         constexpr uint32_t kSide = 4;

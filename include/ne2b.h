@@ -344,6 +344,13 @@ ne2b_status ne2b_fit_ridge_multi(const float *x, uint32_t t, uint32_t f, const u
  * as there).  F at most 32767. */
 ne2b_status ne2b_fit_ridge(const float *x, uint32_t t, uint32_t f, const float *y, float lambda, int device,
                            double *w);
+/* Gives back the memory that the two fits above keep for the next one: up to
+ * 256 MB of each device used (in a memory pool of their own; the device's
+ * default pool is left as it is) and 64 MB of pinned host memory.  Any
+ * thread, any time: what a running fit uses stays with it.  The library does
+ * so itself when a device allocation of its own finds no room.  Call it before
+ * cudaDeviceReset. */
+ne2b_status ne2b_release_workspaces(void);
 
 /* ----------------------------------------------------------- net building */
 /* A host-side network owned by the library, in the ne2b_net_desc layout. */

@@ -137,6 +137,7 @@ _SIGS = {
     "ne2b_create_from_synapses": (C.c_int, [C.POINTER(NetDesc), _p, _u64, _p, _p, _p, _p, C.POINTER(Config), C.c_int,
                                             C.POINTER(_p)]),
     "ne2b_syn_count": (C.c_int, [_p, _pu64]),
+    "ne2b_release_workspaces": (C.c_int, []),
     "ne2b_fit_ridge_multi": (C.c_int, [_p, _u32, _u32, _p, _u32, _f64, C.c_int, _p]),
     "ne2b_batch_fit_ridge_multi": (C.c_int, [_p, _p, _u32, _u32, _p, _u32, _f64, _pu32, _p]),
     "ne2b_fit_ridge": (C.c_int, [_p, _u32, _u32, _p, _f32, C.c_int, _p]),

@@ -12,6 +12,7 @@
 
 #include "ne2b_engine.h"
 #include "ne2b_kernels.h"
+#include "ne2b_workspace.h"
 #include "ne2b_parallel.h"
 
 using ne2b::Engine;
@@ -102,7 +103,7 @@ static ne2b_status create_from_list(ne2b::Engine &eng, const ne2b_net_desc *net,
     };
     auto dalloc = [&](size_t bytes, void **p) -> ne2b_status {
         *p = nullptr;
-        const cudaError_t e = cudaMallocAsync(p, bytes ? bytes : 16, st);
+        const cudaError_t e = device_alloc(p, bytes ? bytes : 16, st);
         if (e != cudaSuccess) return cuda_error(e, "cudaMallocAsync (synapse list)");
         tmp.push_back(*p);
         return NE2B_OK;

@@ -18,6 +18,7 @@
 #include "ne2b_kernels.h"
 #include "ne2b_step_kind.h"
 #include "ne2b_parallel.h"
+#include "ne2b_workspace.h"
 
 namespace ne2b {
 
@@ -501,7 +502,7 @@ ne2b_status Engine::build_net(const ne2b_net_desc *net, const ne2b_config *cfg, 
     auto alloc = [&](void **p, size_t bytes) -> ne2b_status {
         *p = nullptr;
         if (bytes == 0) return NE2B_OK;
-        cudaError_t e = cudaMallocAsync(p, bytes, bst);
+        cudaError_t e = device_alloc(p, bytes, bst);
         if (e != cudaSuccess) return cuda_error(e, "cudaMallocAsync (net arrays)");
         h->allocs.push_back(*p);
         h->dev_bytes += bytes;
@@ -1359,7 +1360,7 @@ ne2b_status Engine::set_input_matrix(NetHost &h, const float *x, uint64_t steps)
     if (steps > 0xffffffffull) return set_error(NE2B_EINVAL, "input matrix longer than 2^32-1 steps");
     const size_t bytes = sizeof(float) * (size_t)steps * h.n_inputs;
     void *p = nullptr;
-    NE2B_CUDA(cudaMallocAsync(&p, bytes, stream_));
+    NE2B_CUDA(device_alloc(&p, bytes, stream_));
     ne2b_status cs = pin_copy(p, x, bytes);
     if (cs == NE2B_OK) cs = pin_close();
     if (cs != NE2B_OK) {
@@ -1754,7 +1755,7 @@ ne2b_status Engine::snapshot(EngineSnapshot &snap) {
     auto grab = [&](void *live, size_t bytes) -> ne2b_status {
         if (!live || !bytes) return NE2B_OK;
         void *b = nullptr;
-        NE2B_CUDA(cudaMallocAsync(&b, bytes, stream_));
+        NE2B_CUDA(device_alloc(&b, bytes, stream_));
         snap.items.push_back({live, b, bytes});
         NE2B_CUDA(cudaMemcpyAsync(b, live, bytes, cudaMemcpyDeviceToDevice, stream_));
         return NE2B_OK;

@@ -445,10 +445,14 @@ __global__ void gather_counts_kernel(const uint16_t *const *__restrict__ win, ui
     }
 }
 
+// A fit's device memory; `device`: of the workspaces kept for that device, or
+// (kEnginePool) of the default pool, as an engine's other arrays.
+constexpr int kEnginePool = -1;
 struct DevBuf {
     std::vector<void *> ps;
     cudaStream_t st;
-    explicit DevBuf(cudaStream_t s) : st(s) {}
+    int device;
+    DevBuf(cudaStream_t s, int dev) : st(s), device(dev) {}
     ~DevBuf() {
         for (void *p : ps) cudaFreeAsync(p, st);
         cudaStreamSynchronize(st);
@@ -456,25 +460,14 @@ struct DevBuf {
     template <class T>
     ne2b_status get(T **p, size_t count) {
         void *q = nullptr;
-        const cudaError_t e = cudaMallocAsync(&q, sizeof(T) * (count ? count : 1), st);
+        const size_t bytes = sizeof(T) * (count ? count : 1);
+        const cudaError_t e = device == kEnginePool ? device_alloc(&q, bytes, st) : workspace_alloc(&q, bytes, device, st);
         if (e != cudaSuccess) return cuda_error(e, "cudaMallocAsync (readout)");
         ps.push_back(q);
         *p = (T *)q;
         return NE2B_OK;
     }
 };
-
-// The default pool keeps up to this much freed memory for the next call
-// (unless it already keeps more): without it each fit maps its workspaces
-// anew.
-void keep_workspace(int device) {
-    cudaMemPool_t pool;
-    uint64_t cur = 0, want = (uint64_t)256 << 20;
-    if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess &&
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &cur) == cudaSuccess && cur < want)
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &want);
-    cudaGetLastError();
-}
 
 // G = U^T U in place of the upper triangle; true when G is positive definite.
 // dblk: scratch, 32 x 32; bad: two flags.
@@ -496,9 +489,9 @@ ne2b_status cholesky(double *g, uint32_t n, double *dblk, unsigned int *bad, cud
 
 // fit_ridge on a device design x[T x F] and host targets y[T].
 ne2b_status fit_binary_on_device(const float *x, uint32_t t, uint32_t f, const float *y_host, float lambda,
-                                 cudaStream_t st, double *w_out) {
+                                 int device, cudaStream_t st, double *w_out) {
     const uint32_t nf = f + 1u;
-    DevBuf buf(st);
+    DevBuf buf(st, device);
     double *a = nullptr, *a0 = nullptr, *b = nullptr;
     float *y = nullptr;
     unsigned int *bad = nullptr;
@@ -559,8 +552,8 @@ ne2b_status check_labels(const uint32_t *labels, uint32_t t, uint32_t f, uint32_
 
 // The fit on a device design x[T x F] (f32) on stream `st`.
 ne2b_status fit_on_device(const float *x, uint32_t t, uint32_t f, const uint32_t *labels, uint32_t k, double lambda,
-                          cudaStream_t st, double *w_out) {
-    DevBuf buf(st);
+                          int device, cudaStream_t st, double *w_out) {
+    DevBuf buf(st, device);
     double *mu = nullptr, *xc = nullptr, *g = nullptr, *a = nullptr, *w = nullptr;
     unsigned int *bad = nullptr;
     NE2B_TRY(buf.get(&mu, f));
@@ -639,10 +632,9 @@ ne2b_status ne2b_fit_ridge_multi(const float *x, uint32_t t, uint32_t f, const u
         cudaStream_t st = nullptr;
         e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
         if (e != cudaSuccess) return ne2b::cuda_error(e, "cudaStreamCreate");
-        ne2b::keep_workspace(device);
         ne2b_status r = NE2B_OK;
         {
-            ne2b::DevBuf buf(st);
+            ne2b::DevBuf buf(st, device);
             const float *xd = x;
             if (!on_device) {
                 float *p = nullptr;
@@ -652,13 +644,18 @@ ne2b_status ne2b_fit_ridge_multi(const float *x, uint32_t t, uint32_t f, const u
                                          "design upload");
                 xd = p;
             }
-            if (r == NE2B_OK) r = ne2b::fit_on_device(xd, t, f, labels, k, lambda, st, w);
+            if (r == NE2B_OK) r = ne2b::fit_on_device(xd, t, f, labels, k, lambda, device, st, w);
         }
         cudaStreamDestroy(st);
         return r;
     } catch (const std::bad_alloc &) {
         return set_error(NE2B_ENOMEM, "host allocation failed");
     }
+}
+
+ne2b_status ne2b_release_workspaces(void) {
+    ne2b::release_workspaces();
+    return NE2B_OK;
 }
 
 }  // extern "C"
@@ -707,14 +704,14 @@ ne2b_status ne2b_batch_fit_ridge_multi(ne2b_batch *b, const uint32_t *nets, uint
                                        double *w) {
     if (!b || !nets || !labels || !w) return set_error(NE2B_EINVAL, "ne2b_batch_fit_ridge_multi: null argument");
     try {
-        ne2b::DevBuf buf(b->eng.stream());
+        ne2b::DevBuf buf(b->eng.stream(), ne2b::kEnginePool);
         float *x = nullptr;
         uint32_t f = 0;
         NE2B_TRY(gather_batch(b, nets, t, windows, buf, &x, &f));
         const ne2b_status cs = ne2b::check_labels(labels, t, f, k);
         if (cs != NE2B_OK) return cs;
         if (n_features) *n_features = f;
-        return ne2b::fit_on_device(x, t, f, labels, k, lambda, b->eng.stream(), w);
+        return ne2b::fit_on_device(x, t, f, labels, k, lambda, ne2b::kEnginePool, b->eng.stream(), w);
     } catch (const std::bad_alloc &) {
         return set_error(NE2B_ENOMEM, "host allocation failed");
     }
@@ -734,10 +731,9 @@ ne2b_status ne2b_fit_ridge(const float *x, uint32_t t, uint32_t f, const float *
         cudaStream_t st = nullptr;
         e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
         if (e != cudaSuccess) return ne2b::cuda_error(e, "cudaStreamCreate");
-        ne2b::keep_workspace(device);
         ne2b_status r = NE2B_OK;
         {
-            ne2b::DevBuf buf(st);
+            ne2b::DevBuf buf(st, device);
             const float *xd = x;
             if (!on_device) {
                 float *p = nullptr;
@@ -747,7 +743,7 @@ ne2b_status ne2b_fit_ridge(const float *x, uint32_t t, uint32_t f, const float *
                                          "design upload");
                 xd = p;
             }
-            if (r == NE2B_OK) r = ne2b::fit_binary_on_device(xd, t, f, y, lambda, st, w);
+            if (r == NE2B_OK) r = ne2b::fit_binary_on_device(xd, t, f, y, lambda, device, st, w);
         }
         cudaStreamDestroy(st);
         return r;
@@ -760,13 +756,13 @@ ne2b_status ne2b_batch_fit_ridge(ne2b_batch *b, const uint32_t *nets, uint32_t t
                                  float lambda, uint32_t *n_features, double *w) {
     if (!b || !nets || !y || !w) return set_error(NE2B_EINVAL, "ne2b_batch_fit_ridge: null argument");
     try {
-        ne2b::DevBuf buf(b->eng.stream());
+        ne2b::DevBuf buf(b->eng.stream(), ne2b::kEnginePool);
         float *x = nullptr;
         uint32_t f = 0;
         NE2B_TRY(gather_batch(b, nets, t, windows, buf, &x, &f));
         if (f >= 32768) return set_error(NE2B_UNSUPPORTED, "fit_ridge: at most 32767 features (F=%u)", f);
         if (n_features) *n_features = f;
-        return ne2b::fit_binary_on_device(x, t, f, y, lambda, b->eng.stream(), w);
+        return ne2b::fit_binary_on_device(x, t, f, y, lambda, ne2b::kEnginePool, b->eng.stream(), w);
     } catch (const std::bad_alloc &) {
         return set_error(NE2B_ENOMEM, "host allocation failed");
     }

@@ -2,8 +2,10 @@
 #include "ne2b_workspace.h"
 
 #include <stdlib.h>
+#include <string.h>
 
 #include <algorithm>
+#include <map>
 #include <mutex>
 
 namespace ne2b {
@@ -11,6 +13,7 @@ namespace {
 
 struct Kept {
     std::mutex mu;
+    std::map<int, cudaMemPool_t> pools;  // by device
     void *pin = nullptr;
     size_t pin_cap = 0;
 };
@@ -19,7 +22,54 @@ Kept &kept() {
     return *k;
 }
 
+cudaMemPool_t fit_pool(int device) {
+    Kept &k = kept();
+    std::lock_guard<std::mutex> lk(k.mu);
+    auto it = k.pools.find(device);
+    if (it != k.pools.end()) return it->second;
+    cudaMemPoolProps props;
+    memset(&props, 0, sizeof props);
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    uint64_t keep = kPoolKeep;
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) cudaGetLastError();
+    k.pools[device] = pool;
+    return pool;
+}
+
 }  // namespace
+
+cudaError_t device_alloc(void **p, size_t bytes, cudaStream_t st) {
+    cudaError_t e = cudaMallocAsync(p, bytes, st);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    release_workspaces();
+    return cudaMallocAsync(p, bytes, st);
+}
+
+cudaError_t workspace_alloc(void **p, size_t bytes, int device, cudaStream_t st) {
+    if (cudaMemPool_t pool = fit_pool(device)) {
+        if (cudaMallocFromPoolAsync(p, bytes, pool, st) == cudaSuccess) return cudaSuccess;
+        cudaGetLastError();
+    }
+    return device_alloc(p, bytes, st);
+}
+
+void release_workspaces() {
+    Kept &k = kept();
+    std::lock_guard<std::mutex> lk(k.mu);
+    for (auto &e : k.pools)
+        if (cudaMemPoolTrimTo(e.second, 0) != cudaSuccess) cudaGetLastError();
+    if (k.pin && cudaFreeHost(k.pin) != cudaSuccess) cudaGetLastError();
+    k.pin = nullptr;
+    k.pin_cap = 0;
+}
 
 void *HostWorkspace::get(size_t bytes) {
     if (bytes <= kPinnedKeep) {

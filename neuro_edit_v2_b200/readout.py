@@ -54,6 +54,12 @@ def fit_ridge(x, y, lam: float, device: int = 0) -> np.ndarray:
     return w
 
 
+def release_workspaces() -> None:
+    """Give back the memory that the fits keep for the next one (up to 256 MB
+    per device and 64 MB of pinned host memory)."""
+    check(lib.ne2b_release_workspaces())
+
+
 def ridge_predict(w: np.ndarray, x) -> np.ndarray:
     """Argmax class per row (the reference's ridge_predict): x @ w[:, :F].T + bias."""
     x = np.asarray(x, dtype=np.float64)

@@ -97,8 +97,10 @@ static ne2b_status create_from_list(ne2b::Engine &eng, const ne2b_net_desc *net,
     const cudaStream_t st = eng.stream();
     const uint32_t n = net->n;
     std::vector<void *> tmp;
+    void *place = nullptr;  // each synapse's place in its row, where there is room for it
     auto release = [&]() {
         for (void *p : tmp) cudaFreeAsync(p, st);
+        if (place) cudaFreeAsync(place, st);
         cudaStreamSynchronize(st);
     };
     auto dalloc = [&](size_t bytes, void **p) -> ne2b_status {
@@ -144,7 +146,6 @@ static ne2b_status create_from_list(ne2b::Engine &eng, const ne2b_net_desc *net,
     if (d_dly) dc.syn.delay_ms = dly; else { LIST_TRY(dalloc(4 * E, &p)); dc.syn.delay_ms = (const float *)p; }
     if (d_kind) dc.syn.kind = kind; else { LIST_TRY(dalloc(n, &p)); dc.syn.kind = (const uint8_t *)p; }
     LIST_TRY(dalloc(2 * E, &p)); dc.steps = (const uint16_t *)p;
-    if (csr_list_short(E)) { LIST_TRY(dalloc(4 * E, &p)); dc.place = (const uint32_t *)p; }
     LIST_TRY(dalloc(4 * (size_t)n, &p)); dc.counts = (const uint32_t *)p;
     LIST_TRY(dalloc(4 * (size_t)n, &p)); dc.cursor = (uint32_t *)p;
     LIST_TRY(dalloc(4 * (size_t)csr_scan_blocks(n), &p)); dc.sums = (uint32_t *)p;
@@ -152,6 +153,18 @@ static ne2b_status create_from_list(ne2b::Engine &eng, const ne2b_net_desc *net,
     LIST_TRY(dalloc(4 * (chunks + 1), &p)); dc.ticket = (uint32_t *)p;
     dc.done = dc.ticket + 1;
     LIST_TRY(dalloc(sizeof(CsrScalars), &p)); dc.sc = (CsrScalars *)p;
+    // last and only where it finds room: the scatter needs none
+    if (E && csr_list_short(E) && device_alloc(&place, 4 * E, st) != cudaSuccess) {
+        cudaGetLastError();
+        place = nullptr;
+    }
+    dc.place = (const uint32_t *)place;
+    auto drop_place = [&]() {
+        if (place) cudaFreeAsync(place, st);
+        place = nullptr;
+        dc.place = nullptr;
+        dc.short_rows = false;
+    };
     dc.syn.n_syn = E;
     dc.syn.n = n;
     dc.syn.dt_ms = cfg->dt_ms;
@@ -186,7 +199,13 @@ static ne2b_status create_from_list(ne2b::Engine &eng, const ne2b_net_desc *net,
     dc.max_delay = sc.max_delay;
     dc.min_delay = sc.min_delay;
     dc.short_rows = dc.place && csr_rows_short(sc.max_row);
-    LIST_TRY(eng.add_net_device_csr(net, cfg, dc, slot));
+    if (!dc.short_rows) drop_place();
+    ne2b_status added = eng.add_net_device_csr(net, cfg, dc, slot);
+    if (added == NE2B_ENOMEM && place) {  // the net may fit without the places
+        drop_place();
+        added = eng.add_net_device_csr(net, cfg, dc, slot);
+    }
+    LIST_TRY(added);
     LIST_TRY(cuda_error(cudaMemcpyAsync(&sc, dc.sc, sizeof sc, cudaMemcpyDeviceToHost, st), "scatter readback"));
     LIST_TRY(cuda_error(cudaStreamSynchronize(st), "device CSR build"));
     release();

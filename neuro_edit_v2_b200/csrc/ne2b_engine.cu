@@ -923,6 +923,13 @@ bool Engine::plan_resident(std::vector<Tile> &tiles, std::vector<uint32_t> &bloc
         block_tiles = bt;
         res_neurons_ = (uint32_t)((m + 3) / 4 * 4);
         res_smem_ = smem;
+        // custom-tau synapses: a buffer for their currents, if the blocks still fit beside it
+        bool custom = false;
+        for (const NetHost *h : nets_) custom |= h && h->nx;
+        const size_t with = smem + xsyn_buffer_bytes(shape_.block);
+        if (custom && with <= 227 * 1024 &&
+            (uint64_t)std::max(0, resident_occupancy(int_ring_, adex_, shape_.block, shape_.npt, with)) * sm_count_ >= blocks)
+            res_smem_ = with;
         res_grid_ = blocks;
         return true;
     }

@@ -186,8 +186,14 @@ __device__ __forceinline__ void defer_deliver(const NetDev &nd, uint32_t rlo, ui
 // lane adds its own neuron's in order.  (A lane walking its own list, one id
 // after another with five dependent scattered loads each, took 41 us per step
 // on 20k neurons with 10 custom synapses each; so 10.8 us, and 6.5 with
-// delivery deferred.)
-constexpr uint32_t kXChunk = 256;
+// delivery deferred.)  In the resident kernel (RES) the neurons' state comes first:
+// without room for `xs` (null) the currents go from lane to lane (20k neurons
+// as above: 8.2 us per step with the buffer, 19.3 without).
+__device__ __forceinline__ uint32_t dynamic_smem_bytes() {
+    uint32_t r;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(r));
+    return r;
+}
 template <bool RES>
 __device__ __forceinline__ void custom_currents(const NetDev &nd, uint32_t tmod, uint32_t p0, uint32_t p1, bool valid,
                                                 float &I, float *xs, uint32_t lane) {
@@ -219,8 +225,17 @@ __device__ __forceinline__ void custom_currents(const NetDev &nd, uint32_t tmod,
                 x[e] = __fadd_rn(x[e], nd.xw[k]);
                 atomicAnd(pend + (k >> 5), ~bit);  // other bits of the word belong to other targets
             }
-            xs[e * 32u + lane] = x[e];
+            if (!RES || xs) xs[e * 32u + lane] = x[e];
             nd.xsyn[k] = __fmul_rn(x[e], dec[e]);
+        }
+        if (RES && !xs) {
+#pragma unroll
+            for (uint32_t e = 0; e < kXChunk / 32; ++e)
+                for (uint32_t j = e * 32u; j < min((e + 1u) * 32u, m); ++j) {
+                    const float xj = __shfl_sync(0xffffffffu, x[e], j & 31u);
+                    if (base + j >= p0 && base + j < p1) I = __fadd_rn(I, xj);
+                }
+            continue;
         }
         __syncwarp();
         for (uint32_t j = max(p0, base); j < min(p1, base + m); ++j) I = __fadd_rn(I, xs[j - base]);
@@ -340,7 +355,8 @@ __device__ __forceinline__ void process_tile(const EngineDev *__restrict__ eng, 
             I = __fadd_rn(sv, ex[q]);
         }
         if (xsyn_on) {
-            custom_currents<RES>(nd, tmod, xp0[q], xp1[q], valid[q], I, xbuf + warp * kXChunk, lane);
+            custom_currents<RES>(nd, tmod, xp0[q], xp1[q], valid[q], I,
+                                 RES && !xbuf ? nullptr : xbuf + warp * kXChunk, lane);
             if (!valid[q]) continue;
         }
         if (has_stim) {
@@ -1068,8 +1084,10 @@ __global__ void __launch_bounds__(BLOCK) resident_kernel(const EngineDev *__rest
     float *ss = su + M;
     uint16_t *stk = reinterpret_cast<uint16_t *>(ss + M);
     uint16_t *spi = stk + M;
+    // the custom currents' buffer, where the launch has room for it (plan_resident)
+    const uint32_t x_off = resident_head_bytes<BLOCK, NPT>() + 16u * M;
+    float *s_x = dynamic_smem_bytes() >= x_off + xsyn_buffer_bytes(BLOCK) ? reinterpret_cast<float *>(smem + x_off) : nullptr;
     __shared__ __align__(16) ParamRow s_ptab[kSmemParamRows];
-    __shared__ float s_x[BLOCK / 32 * kXChunk];
     const ParamRow *ptab = stage_params<BLOCK>(eng, s_ptab);
     const uint32_t t_lo = eng->block_tiles[blockIdx.x], t_hi = eng->block_tiles[blockIdx.x + 1];
 
@@ -1291,10 +1309,12 @@ int StepKind<INT, ADEX>::resident_occupancy(uint32_t block, uint32_t npt, size_t
 #define X(B, P)                                                                                            \
     if (block == B && npt == P) {                                                                          \
         auto *k = resident_kernel<INT, B, P, ADEX>;                                                        \
-        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) \
-            return 0;                                                                                      \
         int b = 0;                                                                                         \
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, B, smem) != cudaSuccess) return 0;        \
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess || \
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, B, smem) != cudaSuccess) {                \
+            cudaGetLastError(); /* does not fit: not an error of the next launch */                        \
+            return 0;                                                                                      \
+        }                                                                                                  \
         return b;                                                                                          \
     }
     NE2B_SHAPES(X)

@@ -34,6 +34,11 @@ __host__ __device__ constexpr uint32_t resident_head_bytes() {
     return (uint32_t)((smem_lists_words<BLOCK, NPT>() + 1) * 4 + 15) / 16 * 16;
 }
 
+// Custom-tau currents that a warp stages at once, and a block's buffer of them
+// (behind the resident kernel's state where there is room).
+constexpr uint32_t kXChunk = 256;
+__host__ __device__ constexpr uint32_t xsyn_buffer_bytes(uint32_t block) { return block / 32u * kXChunk * 4u; }
+
 // Streaming kernel instances: one net with any features, one net without the
 // optional ones (external current, stimulus, records, windows, custom-tau
 // synapses, f32 trace, watches), many nets (batches, the server), and many

@@ -177,7 +177,8 @@ ne2b_status ne2b_set_gauss_noise(ne2b_sim *sim, float sd);                 /* ne
  * cooperative resident kernel (NE2B_UNSUPPORTED when the nets' state does
  * not fit in shared memory; *resident reports whether it runs).  Results are
  * the same (bit for bit with the int32 ring).  The environment variable
- * NE2B_KERNEL=stream|resident sets the initial mode of every handle. */
+ * NE2B_KERNEL=stream|resident sets the initial mode of every sim and batch; a
+ * server heeds stream alone, since its nets come and go. */
 enum { NE2B_KERNEL_AUTO = 0, NE2B_KERNEL_STREAM = 1, NE2B_KERNEL_RESIDENT = 2 };
 ne2b_status ne2b_set_kernel_mode(ne2b_sim *sim, int32_t mode);
 ne2b_status ne2b_kernel_mode(ne2b_sim *sim, int32_t *mode, int32_t *resident);

@@ -768,6 +768,8 @@ ne2b_status ne2b_server_create(const ne2b_server_config *cfg, int device, ne2b_s
         s->cfg = *cfg;
         if (s->cfg.steps_per_launch == 0) s->cfg.steps_per_launch = 64;
         ne2b_status st = s->eng.init(device, cfg->int_weights != 0, cfg->max_requests);
+        // the resident kernel refuses nets past its shared memory; a server's come and go
+        if (st == NE2B_OK && s->eng.mode() == ne2b::kModeResident) st = s->eng.set_mode(ne2b::kModeAuto);
         if (st == NE2B_OK) st = ne2b::cuda_error(cudaStreamCreateWithFlags(&s->rstream, cudaStreamNonBlocking), "result stream");
         for (int k = 0; k < 2 && st == NE2B_OK; ++k)
             st = ne2b::cuda_error(cudaEventCreateWithFlags(&s->step_ev[k], cudaEventDisableTiming), "event");

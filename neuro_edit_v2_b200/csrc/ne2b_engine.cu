@@ -864,9 +864,10 @@ int Engine::step_variant(const TileShape &s) const {
     uint32_t used = 0;
     for (const NetHost *h : nets_)
         if (h) used |= h->dev.flags;
-    if (multi_net) return (used & kDebug) ? kStepMulti : kStepMultiLean;
+    const int xs = (used & kNetXsyn) ? kStepXs : 0;
+    if (multi_net) return (used & kDebug) ? kStepMulti | xs : kStepMultiLean;
     const int ws = ws_applies(s) ? kStepWS : 0;
-    if (stim_tiles_ || (used & (kDebug | kInput))) return kStepSingle | ws;
+    if (stim_tiles_ || (used & (kDebug | kInput))) return kStepSingle | ws | xs;
     return kStepPlain | ws;
 }
 

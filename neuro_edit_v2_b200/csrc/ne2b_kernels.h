@@ -16,7 +16,8 @@ void shape_list(uint32_t *blocks, uint32_t *npts, uint32_t *count);
 // instance of the step kernels runs).  `variant` (StepVariant): kStepMulti
 // when the engine holds many nets (a batch or the server), whose streaming
 // kernel stages several tiles' records and net descriptors ahead; kStepPlain
-// for one net without the optional features; else kStepSingle.
+// for one net without the optional features; else kStepSingle; kStepXs where
+// a net has custom-tau synapses.
 int step_occupancy(bool int_ring, bool adex, int variant, uint32_t block, uint32_t npt);
 // k_step > 0 launches are programmatic (they follow step k_step - 1 of the
 // same launch group); k_step = 0 follows advance_kernel or host copies and

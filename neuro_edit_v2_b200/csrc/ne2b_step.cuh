@@ -693,18 +693,22 @@ __device__ __forceinline__ void stage_net(const EngineDev *__restrict__ eng, uin
 constexpr uint32_t kStageTiles = 16;
 
 // PLAIN: the lean instance; single-net, it also drops the input features
-// (LEAN and NOIO), many-net only the others (LEAN).
-template <bool INT, int BLOCK, int NPT, bool ADEX, bool MULTI, bool PLAIN>
+// (LEAN and NOIO), many-net only the others (LEAN).  XS: some net has
+// custom-tau synapses; the other nets do without that pass (compiled into
+// every instance, it made a recorded net of 200k neurons take 4.7 us per step
+// quiet and 9.1 active; without it 3.0 and 5.9).
+template <bool INT, int BLOCK, int NPT, bool ADEX, bool MULTI, bool PLAIN, bool XS>
 __device__ __forceinline__ void step_body(const EngineDev *__restrict__ eng, uint32_t k_step) {
     pdl_trigger();
     constexpr uint32_t kNetWords = sizeof(NetDev) / 16;
     __shared__ uint32_t s_lists[smem_lists_words<BLOCK, NPT>()];
     __shared__ __align__(16) NetDev s_nd;
     __shared__ __align__(16) ParamRow s_ptab[kSmemParamRows];
-    __shared__ float s_x[PLAIN ? 1 : BLOCK / 32 * kXChunk];
+    __shared__ float s_x[XS ? BLOCK / 32 * kXChunk : 1];
     static_assert(sizeof(NetDev) % 16 == 0 && sizeof(ParamRow) % 16 == 0, "16-byte staging");
     static_assert(kNetWords <= BLOCK && kStageTiles <= BLOCK, "one 16-byte word per thread");
     const SmemLists sl = smem_lists(s_lists, BLOCK * NPT, BLOCK / 32);
+    static_assert(!(XS && PLAIN), "a lean instance has no custom-tau synapses");
     const uint32_t n_tiles = eng->n_tiles;
     if constexpr (!MULTI) {
         uint32_t tix = blockIdx.x;
@@ -719,10 +723,9 @@ __device__ __forceinline__ void step_body(const EngineDev *__restrict__ eng, uin
             const uint64_t t = s_nd.t + k_step;
             uint32_t tmod = s_nd.tmod + k_step;
             if (tmod >= s_nd.D) tmod %= s_nd.D;
-            process_tile<INT, BLOCK, NPT, false, ADEX, false, PLAIN, PLAIN>(eng, ptab, s_nd, tile, t, tmod, k_step,
-                                                             s_nd.v + tile.start, s_nd.u + tile.start,
-                                                             s_nd.s + tile.start, s_nd.tk + tile.start,
-                                                             s_nd.pidx + tile.start, sl, s_x);
+            process_tile<INT, BLOCK, NPT, false, ADEX, false, PLAIN, PLAIN, false, false, XS>(
+                eng, ptab, s_nd, tile, t, tmod, k_step, s_nd.v + tile.start, s_nd.u + tile.start, s_nd.s + tile.start,
+                s_nd.tk + tile.start, s_nd.pidx + tile.start, sl, s_x);
             if (nx >= n_tiles) break;
             const Tile next = eng->tiles[nx];
             if (next.net != tile.net) {
@@ -770,17 +773,16 @@ __device__ __forceinline__ void step_body(const EngineDev *__restrict__ eng, uin
             const uint64_t t = s_nd.t + k_step;
             uint32_t tmod = s_nd.tmod + k_step;
             if (tmod >= s_nd.D) tmod %= s_nd.D;
-            process_tile<INT, BLOCK, NPT, false, ADEX, true, PLAIN>(eng, ptab, s_nd, tile, t, tmod, k_step,
-                                                            s_nd.v + tile.start, s_nd.u + tile.start,
-                                                            s_nd.s + tile.start, s_nd.tk + tile.start,
-                                                            s_nd.pidx + tile.start, sl, s_x);
+            process_tile<INT, BLOCK, NPT, false, ADEX, true, PLAIN, false, false, false, XS>(
+                eng, ptab, s_nd, tile, t, tmod, k_step, s_nd.v + tile.start, s_nd.u + tile.start, s_nd.s + tile.start,
+                s_nd.tk + tile.start, s_nd.pidx + tile.start, sl, s_x);
         }
     }
 }
 
-template <bool INT, int BLOCK, int NPT, bool ADEX, bool MULTI, bool PLAIN>
+template <bool INT, int BLOCK, int NPT, bool ADEX, bool MULTI, bool PLAIN, bool XS>
 __global__ void __launch_bounds__(BLOCK) step_kernel(const EngineDev *__restrict__ eng, uint32_t k_step) {
-    step_body<INT, BLOCK, NPT, ADEX, MULTI, PLAIN>(eng, k_step);
+    step_body<INT, BLOCK, NPT, ADEX, MULTI, PLAIN, XS>(eng, k_step);
 }
 
 // The plain single-net instance at one neuron per thread, held to 64
@@ -792,7 +794,7 @@ __global__ void __launch_bounds__(BLOCK) step_kernel(const EngineDev *__restrict
 template <bool INT, int BLOCK, bool ADEX>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) step_kernel_r64(const EngineDev *__restrict__ eng,
                                                                        uint32_t k_step) {
-    step_body<INT, BLOCK, 1, ADEX, false, true>(eng, k_step);
+    step_body<INT, BLOCK, 1, ADEX, false, true, false>(eng, k_step);
 }
 
 // -------------------------------------- streaming kernel, delivery deferred
@@ -887,7 +889,7 @@ __host__ __device__ constexpr int ws_warps() {
     return BLOCK <= 128 ? 2 : 4;
 }
 
-template <bool INT, int BLOCK, int NPT, bool ADEX, bool PLAIN>
+template <bool INT, int BLOCK, int NPT, bool ADEX, bool PLAIN, bool XS>
 __global__ void __launch_bounds__(BLOCK + 32 * ws_warps<BLOCK>()) step_kernel_ws(const EngineDev *__restrict__ eng,
                                                                                uint32_t k_step) {
     pdl_trigger();
@@ -896,7 +898,7 @@ __global__ void __launch_bounds__(BLOCK + 32 * ws_warps<BLOCK>()) step_kernel_ws
     __shared__ __align__(16) NetDev s_nd;
     __shared__ __align__(16) ParamRow s_ptab[kSmemParamRows];
     __shared__ __align__(16) uint4 s_cell[kWsCells];
-    __shared__ float s_x[PLAIN ? 1 : BLOCK / 32 * kXChunk];
+    __shared__ float s_x[XS ? BLOCK / 32 * kXChunk : 1];
     __shared__ uint32_t s_ctr[4];
     static_assert(sizeof(NetDev) / 16 <= BLOCK, "one 16-byte word per thread");
     const uint32_t n_tiles = eng->n_tiles;
@@ -918,7 +920,7 @@ __global__ void __launch_bounds__(BLOCK + 32 * ws_warps<BLOCK>()) step_kernel_ws
         uint32_t nspk = 0;  // this warp's spikes (warp-uniform)
         const SmemLists none{};
         for (;;) {
-            process_tile<INT, BLOCK, NPT, false, ADEX, false, PLAIN, PLAIN, true>(
+            process_tile<INT, BLOCK, NPT, false, ADEX, false, PLAIN, PLAIN, true, false, XS>(
                 eng, ptab, s_nd, tile, t, tmod, k_step, s_nd.v + tile.start, s_nd.u + tile.start, s_nd.s + tile.start,
                 s_nd.tk + tile.start, s_nd.pidx + tile.start, none, s_x, &wq, &nspk);
             tix += gridDim.x;
@@ -943,7 +945,7 @@ __global__ void __launch_bounds__(BLOCK + 32 * ws_warps<BLOCK>()) step_kernel_ws
     const uint16_t *__restrict__ delay16 = s_nd.delay16;
     const uint32_t n_pad = s_nd.n_pad, D = s_nd.D;
     const bool wide = s_nd.flags & kNetDelayWide;
-    const bool xsyn_on = !PLAIN && (s_nd.flags & kNetXsyn);
+    const bool xsyn_on = XS && (s_nd.flags & kNetXsyn);
     const uint32_t e_total = s_nd.rowptr[s_nd.n];  // a queued row must lie inside the CSR
     const uint64_t pol = ring_policy();
     for (;;) {
@@ -1209,73 +1211,57 @@ static cudaError_t launch_pdl(void (*kernel)(Args...), uint32_t grid, uint32_t b
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// The instance for a tile shape and variant, and its threads per block.
+struct StepInstance {
+    void (*kernel)(const EngineDev *, uint32_t);
+    uint32_t threads;
+};
 template <bool INT, bool ADEX>
-int StepKind<INT, ADEX>::occupancy(uint32_t block, uint32_t npt, int variant) {
-    if (variant & kStepWS) {
-#define X(B, P)                                                                                                 \
-        if (block == B && npt == P) {                                                                           \
-            int b = 0;                                                                                          \
-            if ((variant & ~kStepWS) == kStepPlain)                                                             \
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, step_kernel_ws<INT, B, P, ADEX, true>,        \
-                                                              B + 32 * ws_warps<B>(), 0);                       \
-            else                                                                                                \
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, step_kernel_ws<INT, B, P, ADEX, false>,       \
-                                                              B + 32 * ws_warps<B>(), 0);                       \
-            return b;                                                                                           \
-        }
-        NE2B_WS_SHAPES(X)
-#undef X
-        return 0;
+static StepInstance step_instance(uint32_t block, uint32_t npt, int variant) {
+#define X(B, P)                                                                                \
+    if (block == B && npt == P && (variant & kStepWS)) {                                       \
+        const uint32_t threads = B + 32 * ws_warps<B>();                                       \
+        switch (variant & ~kStepWS) {                                                          \
+            case kStepPlain: return {step_kernel_ws<INT, B, P, ADEX, true, false>, threads};   \
+            case kStepSingle: return {step_kernel_ws<INT, B, P, ADEX, false, false>, threads}; \
+            default: return {step_kernel_ws<INT, B, P, ADEX, false, true>, threads};           \
+        }                                                                                      \
     }
-#define X(B, P)                                                                                                 \
-    if (block == B && npt == P) {                                                                               \
-        int b = 0;                                                                                              \
-        if (variant == kStepMulti)                                                                              \
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, step_kernel<INT, B, P, ADEX, true, false>, B, 0);  \
-        else if (variant == kStepMultiLean)                                                                     \
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, step_kernel<INT, B, P, ADEX, true, true>, B, 0);   \
-        else if (variant == kStepPlain && P == 1)                                                               \
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, step_kernel_r64<INT, B, ADEX>, B, 0);              \
-        else if (variant == kStepPlain)                                                                         \
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, step_kernel<INT, B, P, ADEX, false, true>, B, 0);  \
-        else                                                                                                    \
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, step_kernel<INT, B, P, ADEX, false, false>, B, 0); \
-        return b;                                                                                               \
+    NE2B_WS_SHAPES(X)
+#undef X
+    if (variant & kStepWS) return {nullptr, 0};
+#define X(B, P)                                                                                \
+    if (block == B && npt == P) {                                                              \
+        switch (variant) {                                                                     \
+            case kStepMulti: return {step_kernel<INT, B, P, ADEX, true, false, false>, B};     \
+            case kStepMulti | kStepXs: return {step_kernel<INT, B, P, ADEX, true, false, true>, B}; \
+            case kStepMultiLean: return {step_kernel<INT, B, P, ADEX, true, true, false>, B};  \
+            case kStepPlain:                                                                   \
+                if constexpr (P == 1) return {step_kernel_r64<INT, B, ADEX>, B};               \
+                else return {step_kernel<INT, B, P, ADEX, false, true, false>, B};             \
+            case kStepSingle: return {step_kernel<INT, B, P, ADEX, false, false, false>, B};   \
+            default: return {step_kernel<INT, B, P, ADEX, false, false, true>, B};             \
+        }                                                                                      \
     }
     NE2B_SHAPES(X)
 #undef X
-    return 0;
+    return {nullptr, 0};
+}
+
+template <bool INT, bool ADEX>
+int StepKind<INT, ADEX>::occupancy(uint32_t block, uint32_t npt, int variant) {
+    const StepInstance s = step_instance<INT, ADEX>(block, npt, variant);
+    int b = 0;
+    if (s.kernel) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, s.kernel, (int)s.threads, 0);
+    return b;
 }
 
 template <bool INT, bool ADEX>
 cudaError_t StepKind<INT, ADEX>::launch(uint32_t block, uint32_t npt, int variant, const EngineDev *eng,
                                         uint32_t k_step, uint32_t grid, cudaStream_t st) {
-    if (variant & kStepWS) {
-#define X(B, P)                                                                                                    \
-        if (block == B && npt == P)                                                                                \
-            return (variant & ~kStepWS) == kStepPlain                                                              \
-                       ? launch_pdl(step_kernel_ws<INT, B, P, ADEX, true>, grid, B + 32 * ws_warps<B>(), st,       \
-                                    k_step > 0, eng, k_step)                                                       \
-                       : launch_pdl(step_kernel_ws<INT, B, P, ADEX, false>, grid, B + 32 * ws_warps<B>(), st,      \
-                                    k_step > 0, eng, k_step);
-        NE2B_WS_SHAPES(X)
-#undef X
-        return cudaErrorInvalidValue;
-    }
-#define X(B, P)                                                                                                   \
-    if (block == B && npt == P)                                                                                   \
-        return variant == kStepMulti                                                                              \
-                   ? launch_pdl(step_kernel<INT, B, P, ADEX, true, false>, grid, B, st, k_step > 0, eng, k_step)  \
-               : variant == kStepMultiLean                                                                        \
-                   ? launch_pdl(step_kernel<INT, B, P, ADEX, true, true>, grid, B, st, k_step > 0, eng, k_step)   \
-               : variant == kStepPlain && P == 1                                                                  \
-                   ? launch_pdl(step_kernel_r64<INT, B, ADEX>, grid, B, st, k_step > 0, eng, k_step)              \
-               : variant == kStepPlain                                                                            \
-                   ? launch_pdl(step_kernel<INT, B, P, ADEX, false, true>, grid, B, st, k_step > 0, eng, k_step)  \
-                   : launch_pdl(step_kernel<INT, B, P, ADEX, false, false>, grid, B, st, k_step > 0, eng, k_step);
-    NE2B_SHAPES(X)
-#undef X
-    return cudaErrorInvalidValue;
+    const StepInstance s = step_instance<INT, ADEX>(block, npt, variant);
+    if (!s.kernel) return cudaErrorInvalidValue;
+    return launch_pdl(s.kernel, grid, s.threads, st, k_step > 0, eng, k_step);
 }
 
 template <bool INT, bool ADEX>

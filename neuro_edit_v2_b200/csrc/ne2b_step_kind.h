@@ -51,6 +51,8 @@ enum StepVariant : int { kStepSingle = 0, kStepMulti = 1, kStepPlain = 2, kStepM
 // Added to kStepSingle or kStepPlain: the warp-specialised instance
 // (separate delivery warps; engines of one net, NE2B_WS_SHAPES only).
 constexpr int kStepWS = 0x10;
+// Added to kStepSingle or kStepMulti: some net has custom-tau synapses.
+constexpr int kStepXs = 0x20;
 
 constexpr size_t kClSmemMax = 200 * 1024;  // dynamic shared memory of a cluster kernel block, at most
 constexpr uint32_t kClMaxThreads = 1024;  // threads of a cluster kernel block, at most

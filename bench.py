@@ -412,6 +412,8 @@ def run_ours(args):
     peak, peak_kind = load_peaks()
     achieved = alg_bytes / (launch_ms / 1000.0) / 1e9
     tr = load_traffic()
+    if (tr or {}).get("runs") != tiling["runs"]:
+        tr = None  # the stored capture is of another kernel than the timed one
 
     # active companion regime (same net, Poisson kicks on top)
     act = nb.B200Sim(net, make_cfg(nb, True), device=dev)

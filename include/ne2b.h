@@ -182,6 +182,11 @@ ne2b_status ne2b_set_gauss_noise(ne2b_sim *sim, float sd);                 /* ne
 enum { NE2B_KERNEL_AUTO = 0, NE2B_KERNEL_STREAM = 1, NE2B_KERNEL_RESIDENT = 2 };
 ne2b_status ne2b_set_kernel_mode(ne2b_sim *sim, int32_t mode);
 ne2b_status ne2b_kernel_mode(ne2b_sim *sim, int32_t *mode, int32_t *resident);
+/* The kernel that the next steps run on, with the nets and settings of now:
+ * the streaming kernel, the resident one, thread-block clusters, or the
+ * streaming kernel with deferred delivery. */
+enum { NE2B_RUNS_STREAM = 1, NE2B_RUNS_RESIDENT = 2, NE2B_RUNS_CLUSTER = 3, NE2B_RUNS_DEFERRED = 4 };
+ne2b_status ne2b_running_kernel(ne2b_sim *sim, int32_t *kernel);
 /* Time every (kernel, tile shape, occupancy) candidate on this sim for
  * steps_per_trial steps from a device snapshot of its state and keep the
  * fastest (the state is restored afterwards; AUTO mode may switch kernel). */
@@ -259,6 +264,7 @@ ne2b_status ne2b_batch_dev_mem_bytes(ne2b_batch *b, uint64_t *bytes);
 ne2b_status ne2b_batch_last_step_ms(ne2b_batch *b, float *ms);
 ne2b_status ne2b_batch_set_kernel_mode(ne2b_batch *b, int32_t mode);
 ne2b_status ne2b_batch_kernel_mode(ne2b_batch *b, int32_t *mode, int32_t *resident);
+ne2b_status ne2b_batch_running_kernel(ne2b_batch *b, int32_t *kernel);
 ne2b_status ne2b_batch_stream(ne2b_batch *b, void **stream);
 ne2b_status ne2b_batch_kernel_launches(ne2b_batch *b, uint64_t *launches);
 /* ne2b_fit_ridge_multi on features that stay on the device: trial r is net
@@ -324,6 +330,7 @@ ne2b_status ne2b_server_synchronize(ne2b_server *s);
 /* Tile shape of the server's step kernel (default 128 threads x 1 neuron);
  * same shapes as ne2b_set_tile_shape.  Waits for queued launches. */
 ne2b_status ne2b_server_set_tile_shape(ne2b_server *s, uint32_t block, uint32_t npt, uint32_t blocks_per_sm);
+ne2b_status ne2b_server_running_kernel(ne2b_server *s, int32_t *kernel);
 ne2b_status ne2b_server_stream(ne2b_server *s, void **stream);
 ne2b_status ne2b_server_kernel_launches(ne2b_server *s, uint64_t *launches);
 

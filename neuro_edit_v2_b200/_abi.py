@@ -138,6 +138,9 @@ _SIGS = {
                                             C.POINTER(_p)]),
     "ne2b_syn_count": (C.c_int, [_p, _pu64]),
     "ne2b_release_workspaces": (C.c_int, []),
+    "ne2b_running_kernel": (C.c_int, [_p, C.POINTER(_i32)]),
+    "ne2b_batch_running_kernel": (C.c_int, [_p, C.POINTER(_i32)]),
+    "ne2b_server_running_kernel": (C.c_int, [_p, C.POINTER(_i32)]),
     "ne2b_fit_ridge_multi": (C.c_int, [_p, _u32, _u32, _p, _u32, _f64, C.c_int, _p]),
     "ne2b_batch_fit_ridge_multi": (C.c_int, [_p, _p, _u32, _u32, _p, _u32, _f64, _pu32, _p]),
     "ne2b_fit_ridge": (C.c_int, [_p, _u32, _u32, _p, _f32, C.c_int, _p]),

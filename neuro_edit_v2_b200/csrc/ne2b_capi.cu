@@ -489,6 +489,11 @@ ne2b_status ne2b_tile_shape(ne2b_sim *sim, uint32_t *block, uint32_t *npt, uint3
     return NE2B_OK;
 }
 
+ne2b_status ne2b_running_kernel(ne2b_sim *sim, int32_t *kernel) {
+    if (!sim || !kernel) return set_error(NE2B_EINVAL, "null argument");
+    GUARD(sim->eng.running_kernel(kernel));
+}
+
 ne2b_status ne2b_set_delivery_warps(ne2b_sim *sim, int32_t on) {
     if (!sim) return set_error(NE2B_EINVAL, "null sim handle");
     ne2b::TileShape sh = sim->eng.shape();
@@ -499,9 +504,11 @@ ne2b_status ne2b_set_delivery_warps(ne2b_sim *sim, int32_t on) {
 ne2b_status ne2b_delivery_warps(ne2b_sim *sim, int32_t *on, int32_t *active) {
     if (!sim || !on || !active) return set_error(NE2B_EINVAL, "null argument");
     GUARD(([&]() -> ne2b_status {
+        int32_t runs = 0;
+        const ne2b_status st = sim->eng.running_kernel(&runs);
+        if (st != NE2B_OK) return st;
         *on = sim->eng.shape().ws ? 1 : 0;
-        *active = (!sim->eng.resident() && !sim->eng.cluster() && !sim->eng.deferred() &&
-                   sim->eng.ws_applies(sim->eng.shape())) ? 1 : 0;
+        *active = runs == NE2B_RUNS_STREAM && sim->eng.ws_applies(sim->eng.shape()) ? 1 : 0;
         return NE2B_OK;
     })());
 }
@@ -686,6 +693,11 @@ ne2b_status ne2b_batch_stream(ne2b_batch *b, void **stream) {
     if (!b || !stream) return set_error(NE2B_EINVAL, "null argument");
     *stream = (void *)b->eng.stream();
     return NE2B_OK;
+}
+
+ne2b_status ne2b_batch_running_kernel(ne2b_batch *b, int32_t *kernel) {
+    if (!b || !kernel) return set_error(NE2B_EINVAL, "null argument");
+    GUARD(b->eng.running_kernel(kernel));
 }
 
 ne2b_status ne2b_batch_kernel_launches(ne2b_batch *b, uint64_t *launches) {
@@ -1102,6 +1114,11 @@ ne2b_status ne2b_selftest_barrier_timeout(int device, uint32_t limit_ms, int32_t
 ne2b_status ne2b_server_synchronize(ne2b_server *s) {
     if (!s) return set_error(NE2B_EINVAL, "null server handle");
     GUARD(s->eng.sync());
+}
+
+ne2b_status ne2b_server_running_kernel(ne2b_server *s, int32_t *kernel) {
+    if (!s || !kernel) return set_error(NE2B_EINVAL, "null argument");
+    GUARD(s->eng.running_kernel(kernel));
 }
 
 ne2b_status ne2b_server_stream(ne2b_server *s, void **stream) {

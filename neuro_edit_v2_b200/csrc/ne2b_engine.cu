@@ -1051,6 +1051,13 @@ ne2b_status Engine::choose_kernel() {
     return NE2B_OK;
 }
 
+ne2b_status Engine::running_kernel(int32_t *kernel) {
+    NE2B_CUDA(cudaSetDevice(device_));
+    NE2B_TRY(choose_kernel());
+    *kernel = resident_ ? NE2B_RUNS_RESIDENT : cluster_ ? NE2B_RUNS_CLUSTER : defer_ ? NE2B_RUNS_DEFERRED : NE2B_RUNS_STREAM;
+    return NE2B_OK;
+}
+
 // One launch per cluster size, side by side on their own streams, forked
 // from and joined to the engine's stream.
 ne2b_status Engine::launch_clusters(uint32_t steps) {

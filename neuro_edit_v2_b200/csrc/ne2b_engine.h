@@ -229,9 +229,7 @@ class Engine {
     uint64_t launches() const { return launches_; }
     void count_launches(uint64_t k) { launches_ += k; }  // kernels launched by entry points outside the engine
     bool resident() const { return resident_; }
-    // the cluster kernel runs the next steps (ne2b_cluster.cuh)
-    bool cluster() { return choose_kernel() == NE2B_OK && cluster_; }
-    bool deferred() { return choose_kernel() == NE2B_OK && defer_; }
+    ne2b_status running_kernel(int32_t *kernel);  // NE2B_RUNS_*
     int mode() const { return mode_; }
     ne2b_status set_mode(int m);
     // the streaming kernel runs separate delivery warps for shape `s`

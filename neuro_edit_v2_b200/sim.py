@@ -44,6 +44,15 @@ def _list_array(a, dtype):
     return len(a), a.ctypes.data, a
 
 
+RUNS = {1: "stream", 2: "resident", 3: "cluster", 4: "deferred"}
+
+
+def _running(entry, handle) -> str:
+    k = C.c_int32()
+    check(entry(handle, C.byref(k)))
+    return RUNS[int(k.value)]
+
+
 class B200Sim:
     """One network on one B200: `Backend` with kind B200."""
 
@@ -313,12 +322,19 @@ class B200Sim:
         check(lib.ne2b_delivery_warps(self._h, C.byref(a), C.byref(b)))
         return bool(a.value), bool(b.value)
 
+    def running_kernel(self) -> str:
+        """The kernel that the next steps run on."""
+        return _running(lib.ne2b_running_kernel, self._h)
+
     def tiling(self) -> dict:
+        """The step kernel's settings ("kernel", "block", ...: the streaming
+        or resident kernel and its tiles) and the kernel that runs ("runs":
+        on "cluster" the tiles do not apply, on "deferred" they are 128 x 1)."""
         a, b, c = C.c_uint32(), C.c_uint32(), C.c_uint32()
         check(lib.ne2b_tile_shape(self._h, C.byref(a), C.byref(b), C.byref(c)))
         return {"kernel": "resident" if self.kernel_mode()[1] else "stream", "block": int(a.value),
                 "neurons_per_thread": int(b.value), "blocks_per_sm": int(c.value),
-                "delivery_warps": self.delivery_warps()[1]}
+                "delivery_warps": self.delivery_warps()[1], "runs": self.running_kernel()}
 
     # --- instrumentation (new) ------------------------------------------
     def stream_handle(self) -> int:
@@ -345,7 +361,7 @@ class B200Sim:
 
 
 class Batch:
-    """Many independent networks stepped together in one kernel per step."""
+    """Many independent networks stepped together."""
 
     def __init__(self, nets, cfgs, device: int = 0):
         self._nets = list(nets)
@@ -450,6 +466,10 @@ class Batch:
     def set_kernel_mode(self, mode: int) -> None:
         check(lib.ne2b_batch_set_kernel_mode(self._h, mode))
 
+    def running_kernel(self) -> str:
+        """The kernel that the next steps run on."""
+        return _running(lib.ne2b_batch_running_kernel, self._h)
+
     def kernel_mode(self) -> tuple[int, bool]:
         m, r = C.c_int32(), C.c_int32()
         check(lib.ne2b_batch_kernel_mode(self._h, C.byref(m), C.byref(r)))
@@ -506,6 +526,10 @@ class Server:
 
     def synchronize(self) -> None:
         check(lib.ne2b_server_synchronize(self._h))
+
+    def running_kernel(self) -> str:
+        """The kernel that the next steps run on, with the requests of now."""
+        return _running(lib.ne2b_server_running_kernel, self._h)
 
     def set_tile_shape(self, block: int, npt: int, blocks_per_sm: int = 0) -> None:
         check(lib.ne2b_server_set_tile_shape(self._h, block, npt, blocks_per_sm))

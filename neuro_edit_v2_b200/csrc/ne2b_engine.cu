@@ -155,6 +155,7 @@ ne2b_status Engine::init(int device, bool int_ring, uint32_t max_nets) {
     NE2B_CUDA(cudaMalloc(&d_barrier_, 2 * sizeof(unsigned int)));
     NE2B_CUDA(cudaMemset(d_barrier_, 0, 2 * sizeof(unsigned int)));
     d_err_ = d_barrier_ + 1;
+    NE2B_CUDA(cudaMalloc(&d_plan_, sizeof(ClusterNet) * nets_cap_));
     if (const char *pdl = getenv("NE2B_PDL")) set_pdl(strcmp(pdl, "0") != 0);
     if (const char *m = getenv("NE2B_KERNEL")) {
         if (!strcmp(m, "stream")) mode_ = kModeStream;
@@ -959,7 +960,8 @@ int Engine::resident_clusters(const ClusterClass &k) {
 // takes the smallest power of two of blocks, at most 16) and `per_thread`
 // neurons per thread; returns the share of the device that they fill at
 // once, or a negative number when one does not fit.
-double Engine::cluster_classes(uint32_t per_block, uint32_t per_thread, std::vector<ClusterNet> &plan) {
+// `*us`: the estimated time of a step, see plan_cluster.
+double Engine::cluster_classes(uint32_t per_block, uint32_t per_thread, std::vector<ClusterNet> &plan, double *us) {
     classes_.clear();
     plan.clear();
     // by cluster size, kind of hop and threads (in octaves), the largest first
@@ -971,9 +973,10 @@ double Engine::cluster_classes(uint32_t per_block, uint32_t per_thread, std::vec
         while ((32ull * per_thread << (c + octave)) < h->n_pad) ++octave;
         by[{c, h->dev.hop > 1u ? 1u : 0u, octave}].push_back(h);
     }
-    double filled = 0.0;
+    double filled = 0.0, slowest = 0.0, queued = 0.0;
     for (auto &e : by) {
         ClusterClass k{};
+        bool adex = false;
         k.blocks = 1u << e.first[0];
         k.first = (uint32_t)plan.size();
         uint32_t most = 0, hop = 1;
@@ -981,6 +984,7 @@ double Engine::cluster_classes(uint32_t per_block, uint32_t per_thread, std::vec
             const uint32_t m = ((h->n_pad + k.blocks - 1) / k.blocks + 31) / 32 * 32;
             most = std::max(most, m);
             hop = std::max(hop, h->dev.hop);
+            adex |= (h->dev.flags & kNetHasAdex) != 0u;
             plan.push_back(ClusterNet{h->slot, m});
         }
         k.count = (uint32_t)e.second.size();
@@ -992,8 +996,26 @@ double Engine::cluster_classes(uint32_t per_block, uint32_t per_thread, std::vec
         if (fit < 1) return -1.0;
         filled += (double)k.count / fit;
         classes_.push_back(k);
+        const double passes = (double)((most + k.shape.threads - 1) / k.shape.threads);
+        const double beside = k.shape.threads <= kClMaxThreads / 2u && filled > 0.5 ? kClMaxThreads / k.shape.threads : 1;
+        const double t = k.shape.one ? (adex ? 1.45 : 1.0) * passes + 0.7 + 0.45e-3 * most * std::min(beside, 4.0)
+                                     : ((adex ? 1.1 : 0.58) * passes + 0.5) * (beside > 1.0 ? 1.5 : 1.0);
+        slowest = std::max(slowest, t);
+        queued += (double)k.count / fit * t;
     }
+    *us = std::max(slowest, queued);
     return filled;
+}
+
+// The same for the streaming kernel, all nets together: a line over the waves
+// of 1024 neurons per SM, within the first and past it, for tiles of up to 128
+// neurons (the server's) and larger ones.
+double Engine::stream_estimate(uint64_t neurons) const {
+    const double waves = (double)neurons / (1024.0 * sm_count_);
+    const bool small = shape_.block * shape_.npt <= 128u, first = waves <= (small || adex_ ? 1.0 : 1.4);
+    if (small)
+        return adex_ ? (first ? 3.1 + 1.3 * waves : 2.6 + 3.2 * waves) : (first ? 2.7 + 1.0 * waves : 2.4 + 2.4 * waves);
+    return adex_ ? (first ? 3.9 + 1.1 * waves : 3.3 + 3.4 * waves) : (first ? 3.2 + 1.1 * waves : 2.9 + 2.1 * waves);
 }
 
 // Cluster plan: each net on one cluster of 1-16 blocks; nets with the same
@@ -1008,9 +1030,26 @@ double Engine::cluster_classes(uint32_t per_block, uint32_t per_thread, std::vec
 // 17-22 ms with blocks of 256 or 512.  One net alone takes a cluster up to
 // 16 x 1024 neurons: at 16,000 the step takes 0.76 us against the streaming
 // kernel's 1.84 (active: 2.5 / 3.7; AdEx 1.3 / 2.3, active 3.3 / 4.5), at
-// 24,000, in two passes, 1.8 / 1.95 (3.9 / 3.8; 2.9 / 2.5; 5.2 / 4.6).  False
-// when a tile shape or a kernel was asked for, or a net is too large or has
-// synapses with their own tau.
+// 24,000, in two passes, 1.8 / 1.95 (3.9 / 3.8; 2.9 / 2.5; 5.2 / 4.6).
+//
+// Several nets: a net is bound to its 16 SMs at most, while the streaming
+// kernel spreads all of them over the device, so clusters lose where a few
+// nets with synapses of delay 1 need many passes.  The plan is compared with
+// the streaming kernel by estimates fitted to the mean of a quiet and an
+// active (25 Hz) step of 2 to 64 equal nets of 8k to 60k neurons.  Measured,
+// clusters / streaming at 256 x 2, mean of both in us: delay 1, 2 x 8k 1.6 /
+// 3.3, 4 x 16k 2.0 / 3.8, 2 x 32k 3.3 / 3.9, 2 x 45k 4.4 / 4.0, 2 x 60k 5.8 /
+// 4.2, 8 x 60k 11.1 / 9.7; delay 6, 2 x 43k 2.2 / 4.2, 48 liquids 6.0 / 11.8, 256
+// liquids in waves 27 / 49.
+// A server (small tiles, fixed_grid) stops at two neurons per thread: of its
+// mixed requests few are busy at a time, and a busy net among many sharing
+// SMs waits longest (64 requests: 510 ms without this limit, 400 with it, 390
+// streaming).  Its requests with local wiring gain more in bursts than the
+// estimate says, so up to 1.15 times the streaming estimate is accepted (12
+// requests: 69-136 ms on clusters, 102-192 streaming).
+//
+// False when a tile shape or a kernel was asked for, or a net is too large or
+// has synapses with their own tau.
 bool Engine::plan_cluster(std::vector<ClusterNet> &plan) {
     classes_.clear();
     if (mode_ != kModeAuto || shape_set_) return false;
@@ -1023,15 +1062,19 @@ bool Engine::plan_cluster(std::vector<ClusterNet> &plan) {
             largest = std::max(largest, h->n_pad);
         }
     if (!total || largest > 16u * (active_nets() > 1 ? kClMaxNeurons : kClMaxThreads)) return false;
-    for (uint32_t per_block = kClMinNeurons; per_block <= 2048u; per_block *= 2u) {
-        const double filled = cluster_classes(per_block, 1u, plan);
-        if (filled > 0.0 && filled <= 1.0) return true;
-    }
-    for (uint32_t per_thread = 2; per_thread <= 8u; ++per_thread) {
-        const double filled = cluster_classes(2048u, per_thread, plan);
-        if (filled > 0.0 && filled <= 1.0) return true;
-    }
-    return cluster_classes(2048u, 4u, plan) > 0.0;  // in waves
+    double us = 0.0;
+    auto plan_that_fits = [&]() -> bool {
+        for (uint32_t per_block = kClMinNeurons; per_block <= 2048u; per_block *= 2u) {
+            const double filled = cluster_classes(per_block, 1u, plan, &us);
+            if (filled > 0.0 && filled <= 1.0) return true;
+        }
+        for (uint32_t per_thread = 2; per_thread <= (fixed_grid ? 2u : 8u); ++per_thread) {
+            const double filled = cluster_classes(2048u, per_thread, plan, &us);
+            if (filled > 0.0 && filled <= 1.0) return true;
+        }
+        return !fixed_grid && cluster_classes(2048u, 4u, plan, &us) > 0.0;  // in waves
+    };
+    return plan_that_fits() && (active_nets() == 1 || us <= (fixed_grid ? 1.15 : 1.0) * stream_estimate(total));
 }
 
 // The plan is made when steps are next run: nets may come and go in between.
@@ -1042,7 +1085,6 @@ ne2b_status Engine::choose_kernel() {
     if (!cluster_ && !resident_) NE2B_TRY(plan_defer());
     if (defer_) NE2B_TRY(build_tiles(defer_shape_));
     if (cluster_) {
-        if (!d_plan_) NE2B_CUDA(cudaMalloc(&d_plan_, sizeof(ClusterNet) * nets_cap_));
         // pageable source, staged by the runtime before the call returns
         NE2B_CUDA(cudaMemcpyAsync(d_plan_, plan.data(), sizeof(ClusterNet) * plan.size(), cudaMemcpyHostToDevice,
                                   stream_));

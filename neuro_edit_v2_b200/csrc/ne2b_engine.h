@@ -260,7 +260,8 @@ class Engine {
         ClusterShape shape;
     };
     int resident_clusters(const ClusterClass &k);
-    double cluster_classes(uint32_t per_block, uint32_t per_thread, std::vector<ClusterNet> &plan);
+    double cluster_classes(uint32_t per_block, uint32_t per_thread, std::vector<ClusterNet> &plan, double *us);
+    double stream_estimate(uint64_t neurons) const;
     bool plan_cluster(std::vector<ClusterNet> &plan);
     ne2b_status launch_clusters(uint32_t steps);
     bool plan_resident(std::vector<Tile> &tiles, std::vector<uint32_t> &block_tiles);

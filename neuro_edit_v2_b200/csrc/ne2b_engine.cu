@@ -1108,25 +1108,34 @@ ne2b_status Engine::launch_clusters(uint32_t steps) {
         full |= h && (h->dev.flags & (kNetRecord | kNetWatch | kNetGridWatch | kNetTraceF32));
     const size_t nc = classes_.size();
     while (nc > 1 && cl_ev_.size() < nc) {
-        cl_ev_.push_back(nullptr);
-        NE2B_CUDA(cudaEventCreateWithFlags(&cl_ev_.back(), cudaEventDisableTiming));
+        cudaEvent_t ev = nullptr;
+        NE2B_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        cl_ev_.push_back(ev);
     }
     while (cl_stream_.size() + 1 < nc) {
-        cl_stream_.push_back(nullptr);
-        NE2B_CUDA(cudaStreamCreateWithFlags(&cl_stream_.back(), cudaStreamNonBlocking));
+        cudaStream_t st = nullptr;
+        NE2B_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+        cl_stream_.push_back(st);
     }
     if (nc > 1) NE2B_CUDA(cudaEventRecord(cl_ev_[0], stream_));
-    for (size_t c = 0; c < nc; ++c) {
+    cudaError_t failed = cudaSuccess;
+    for (size_t c = 0; c < nc && failed == cudaSuccess; ++c) {
         const ClusterClass &k = classes_[c];
         cudaStream_t st = c == 0 ? stream_ : cl_stream_[c - 1];
-        if (c) NE2B_CUDA(cudaStreamWaitEvent(st, cl_ev_[0], 0));
-        NE2B_CUDA(launch_cluster(int_ring_, adex_, full, k.blocks, k.count, k.shape, k.smem, d_eng_,
-                                 d_plan_ + k.first, steps, st));
-        if (c) NE2B_CUDA(cudaEventRecord(cl_ev_[c], st));
+        if (c) failed = cudaStreamWaitEvent(st, cl_ev_[0], 0);
+        if (failed == cudaSuccess)
+            failed = launch_cluster(int_ring_, adex_, full, k.blocks, k.count, k.shape, k.smem, d_eng_,
+                                    d_plan_ + k.first, steps, st);
+        if (failed == cudaSuccess) ++launches_;
     }
-    for (size_t c = 1; c < nc; ++c) NE2B_CUDA(cudaStreamWaitEvent(stream_, cl_ev_[c], 0));
-    launches_ += nc;
-    return NE2B_OK;
+    // joined also when a launch failed: what the others use is freed in the order of stream_
+    for (size_t c = 1; c < nc; ++c) {
+        cudaError_t e = cudaEventRecord(cl_ev_[c], cl_stream_[c - 1]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(stream_, cl_ev_[c], 0);
+        if (e != cudaSuccess) cudaStreamSynchronize(cl_stream_[c - 1]);
+        if (failed == cudaSuccess) failed = e;
+    }
+    return cuda_error(failed, "cluster launch");
 }
 
 // Delivery blocks of the deferred-delivery kernel for a net of n neurons:

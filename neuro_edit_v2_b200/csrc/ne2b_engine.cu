@@ -1876,13 +1876,23 @@ void Engine::drop(EngineSnapshot &snap) {
 ne2b_status Engine::autotune(uint32_t steps_per_trial) {
     if (steps_per_trial == 0) steps_per_trial = graph_steps;
     // what the automatic choice allocates has to be there before the snapshot
+    const bool had_shape = shape_set_;
+    EngineSnapshot snap;
+    ne2b_status ready = NE2B_OK;
     if (mode_ == kModeAuto) {
         shape_set_ = false;
-        NE2B_TRY(rebuild_tiles());
-        NE2B_TRY(choose_kernel());
+        ready = rebuild_tiles();
+        if (ready == NE2B_OK) ready = choose_kernel();
     }
-    EngineSnapshot snap;
-    NE2B_TRY(snapshot(snap));
+    if (ready == NE2B_OK) ready = snapshot(snap);
+    if (ready != NE2B_OK) {  // the sim goes on with the shape that was asked for
+        drop(snap);
+        if (had_shape != shape_set_) {
+            shape_set_ = had_shape;
+            rebuild_tiles();
+        }
+        return ready;
+    }
     // bring the clocks up from idle and size the trials: every candidate runs
     // at least ~3 ms of steps, twice, and keeps its faster repetition
     {

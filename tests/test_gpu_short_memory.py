@@ -17,23 +17,24 @@ REFUSER = r"""
 #include <stdlib.h>
 #include <string.h>
 typedef int (*alloc_fn)(void **, size_t, void *);
-/* REFUSE="bytes:times,bytes:times" */
+/* REFUSE="bytes:times:after,..." : so many, after so many that are served */
 int cudaMallocAsync(void **p, size_t n, void *st) {
     static alloc_fn real;
     static size_t size[8];
-    static int left[8], count = -1;
+    static int left[8], after[8], count = -1;
     if (!real) real = (alloc_fn)dlsym(RTLD_NEXT, "cudaMallocAsync");
     if (count < 0) {
         count = 0;
         const char *s = getenv("REFUSE");
-        while (s && *s && count < 8 && sscanf(s, "%zu:%d", &size[count], &left[count]) == 2) {
+        while (s && *s && count < 8 && sscanf(s, "%zu:%d:%d", &size[count], &left[count], &after[count]) >= 2) {
             ++count;
             s = strchr(s, ',');
             if (s) ++s;
         }
     }
     for (int k = 0; k < count; ++k)
-        if (size[k] == n && left[k] > 0) {
+        if (size[k] == n && after[k] > 0) --after[k];
+        else if (size[k] == n && left[k] > 0) {
             --left[k];
             fprintf(stderr, "refused %zu\n", n);
             return 2; /* cudaErrorMemoryAllocation */
@@ -82,3 +83,34 @@ def test_the_net_is_built_without_the_optional_memory(refuser, sizes):
     r = subprocess.run([sys.executable, "-c", CHILD], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
     assert all(f"refused {s}" in r.stderr for s in sizes)
+
+
+TUNE = r"""
+import torch
+import numpy as np
+import neuro_edit_v2_b200 as nb
+net = nb.random_kout(5000, 20, 3)
+sims = [nb.B200Sim(net, int_weights=1, noise_rate_hz=300.0) for _ in range(2)]
+for s in sims:
+    s.run_steps(50)
+a = sims[1]
+a.set_tile_shape(256, 4)
+try:
+    a.autotune(64)
+except nb.Ne2bError as e:
+    assert "ENOMEM" in str(e)
+    print("refused")
+t = a.tiling()
+assert (t["runs"], t["block"], t["neurons_per_thread"]) == ("stream", 256, 4), t
+for s in sims:
+    s.run_steps(300)
+assert np.array_equal(a.v().view(np.uint32), sims[0].v().view(np.uint32)) and a.spikes_total() > 0
+print("ok")
+"""
+
+
+def test_autotune_without_room_for_its_snapshot_keeps_the_tile_shape(refuser):
+    # 8 bytes per neuron: the lifetime counts, allocated with each sim and then by the snapshot
+    env = dict(os.environ, LD_PRELOAD=refuser, REFUSE=f"{8 * 5056}:2:2")  # 5000 neurons in whole words of 64
+    r = subprocess.run([sys.executable, "-c", TUNE], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.split() == ["refused", "ok"], r.stdout + r.stderr

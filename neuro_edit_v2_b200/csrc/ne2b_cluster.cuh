@@ -3,8 +3,8 @@
 //
 // A net of up to a few tens of thousands of neurons runs on one cluster of
 // 1 to 16 blocks.  Each block owns a contiguous range of the net's neurons
-// whose state (v, u, s, tk, pidx: 16 bytes per neuron) stays in its shared
-// memory for the whole launch; the steps are separated by the hardware's
+// whose state stays in its registers for the whole launch, or, past a neuron
+// per thread, in its shared memory (16 bytes per neuron); the steps are separated by the hardware's
 // cluster barrier, which costs a fraction of a kernel boundary or of a
 // software grid barrier.  Nets of an engine share nothing, so the clusters
 // of a batch or of the server run on without waiting for one another.

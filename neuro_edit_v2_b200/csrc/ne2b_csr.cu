@@ -4,8 +4,7 @@
 //   1. prepass: every synapse's references are checked (the first bad index
 //      is kept), its delay rounded to steps (max(1, roundf(ms / dt)), at most
 //      65535: network.rs:660-666), the largest delay found, and the synapses
-//      counted per source;
-//      per source; the count's atomic add also gives the synapse a place of
+//      counted per source; the count's atomic add also gives the synapse a place of
 //      its own in its row, in no particular order;
 //   2. the counts are scanned into the row pointers;
 //   3. place: every synapse's finished record (target, Dale-signed weight

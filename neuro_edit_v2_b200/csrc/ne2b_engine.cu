@@ -1028,9 +1028,9 @@ double Engine::stream_estimate(uint64_t neurons) const {
 // neurons, 1500 steps: 15.1 ms with blocks of 2048 and five neurons per thread
 // (0.96 of the device), 17-20 ms with one to four (1.4-4 times the device),
 // 17-22 ms with blocks of 256 or 512.  One net alone takes a cluster up to
-// 16 x 1024 neurons: at 16,000 the step takes 0.76 us against the streaming
-// kernel's 1.84 (active: 2.5 / 3.7; AdEx 1.3 / 2.3, active 3.3 / 4.5), at
-// 24,000, in two passes, 1.8 / 1.95 (3.9 / 3.8; 2.9 / 2.5; 5.2 / 4.6).
+// 16 x 1024 neurons: at 16,000 the step takes 0.79 us against the streaming
+// kernel's 1.54 at its best tiles (active: 2.6 / 3.1; AdEx 1.34 / 1.75, active
+// 3.0 / 3.4), at 24,000, in two passes, 1.8 / 1.95 (3.9 / 3.8; 2.9 / 2.5; 5.2 / 4.6).
 //
 // Several nets: a net is bound to its 16 SMs at most, while the streaming
 // kernel spreads all of them over the device, so clusters lose where a few

@@ -45,7 +45,7 @@ __global__ void trace_kernel(const uint16_t *tk, const float *tab, uint32_t n, f
 // takes 32 record words (1024 neurons); warp w adds rows w, w + 32, ... with
 // each lane holding one word, whose 32 bits it adds into a 32-bit counter per
 // bit kept as eight planes of byte counters (a mask and an add for every four
-// bits), emptied into the block's totals in shared memory every 255 rows.
+// bits), emptied into the block's totals in shared memory every 252 rows.
 // Bound by the record's bytes from L2.  (A thread per neuron, one 64-bit
 // modulo and one shared word per row, took 0.2 ms more for 500 rows of 100k
 // neurons.)

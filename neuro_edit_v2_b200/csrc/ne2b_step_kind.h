@@ -75,7 +75,7 @@ struct StepKind {
     static cudaError_t launch_defer(int variant, const EngineDev *eng, uint32_t n_deliver, uint32_t k_step, uint32_t grid, cudaStream_t st);
     static cudaError_t launch_defer_flush(const EngineDev *eng, uint32_t n_deliver, uint32_t steps, cudaStream_t st);
     // cluster kernel: `clusters` clusters of `blocks` blocks; `full` = with
-    // records, custom-tau synapses, f32 trace and watches
+    // records, the f32 trace and watches (custom-tau nets do not run on it)
     static int cluster_fit(bool full, uint32_t blocks, const ClusterShape &cs, size_t smem);
     static cudaError_t launch_cluster(bool full, uint32_t blocks, uint32_t clusters, const ClusterShape &cs,
                                       size_t smem, const EngineDev *eng, const ClusterNet *plan, uint32_t steps,

@@ -35,6 +35,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <exception>
 #include <vector>
 
 #include "ne2b_engine.h"
@@ -654,8 +655,12 @@ ne2b_status ne2b_fit_ridge_multi(const float *x, uint32_t t, uint32_t f, const u
 }
 
 ne2b_status ne2b_release_workspaces(void) {
-    ne2b::release_workspaces();
-    return NE2B_OK;
+    try {
+        ne2b::release_workspaces();
+        return NE2B_OK;
+    } catch (const std::exception &e) {
+        return set_error(NE2B_ENOMEM, "ne2b_release_workspaces: %s", e.what());
+    }
 }
 
 }  // extern "C"
